@@ -175,22 +175,35 @@ __device__ __forceinline__ bool begin_voxel(const PhaseConst<NS>& pc, const doub
 }
 
 // one integrateStress (integrateStateFPI:626-629); returns its Newton iterations
-template <int NS>
-__device__ __forceinline__ int stress_voxel(const PhaseConst<NS>& pc, const SysConst* __restrict__ sc, double* xs,
+template <int NS, class Shape, class SC>
+__device__ __forceinline__ int stress_voxel(const PhaseConst<NS>& pc, const SC* __restrict__ sc, double* xs,
                                             const Numerics& nm, const Fields& f, const PassWork& w, int64_t v,
                                             double dt) {
   const int64_t N = f.N;
   int dnewton = 0;
-  const double step = w.sub[N + v];
-  double Lp[9];
+  // every load of the voxel at once (one exposure of the memory latency), the substep's Fp0
+  // speculatively that of the first substep (see sub_start)
+  const double frac = w.sub[v], step = w.sub[N + v];
+  double Lp[9], F[9], Fp0[9], xi[NS];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) Lp[k] = f.Lp[k * N + v];
+  for (int k = 0; k < 9; ++k) {
+    Lp[k] = f.Lp[k * N + v];
+    F[k] = w.Fs[k * N + v];
+    Fp0[k] = f.Fp0[k * N + v];
+  }
 #pragma unroll
-  for (int s = 0; s < NS; ++s) xs[s * pass_threads<NS>()] = 1.0 / f.state[s * N + v];
+  for (int s = 0; s < NS; ++s) xi[s] = f.state[s * N + v];
+  const double* Fp0g = f.Fp0 + v;
+  if (frac != 0.0) {
+    Fp0g = w.Fp0s + v;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Fp0[k] = Fp0g[k * N];
+  }
+#pragma unroll
+  for (int s = 0; s < NS; ++s) xs[s * Shape::threads] = 1.0 / xi[s];
   double S[6], Fp[9], P[9], Fe[9];
-  const double* Fp0s = (w.sub[v] == 0.0 ? f.Fp0 : w.Fp0s) + v;   // subFp0 (see sub_start)
-  const int st = integrate_stress<NS>(pc, sc, nm, w.Fs + v, Fp0s, N, xs, step * dt, Lp, S, Fp, P, Fe,
-                                      dnewton, w.adg + v, w.lo + v, w.dl + v);
+  const int st = integrate_stress<NS, Shape>(pc, sc, nm, F, Fp0, Fp0g, N, xs, step * dt, Lp, S, Fp, P, Fe, dnewton,
+                                             w.adg + v);
   if (st == 0) {
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
@@ -204,9 +217,10 @@ __device__ __forceinline__ int stress_voxel(const PhaseConst<NS>& pc, const SysC
   }
   w.ctl[v] = st == 0 ? PH_DOT1 : PH_CTRL;
   w.ctl[N + v] = st;
-  w.ctl[2 * N + v] += 1;                                 // state iteration of this substep
-  w.ctl[4 * N + v] += 1;                                 // state iterations, total
-  w.ctl[5 * N + v] += dnewton;                           // Newton iterations, total
+  // without a result: the thread does not wait for them
+  atomicAdd(&w.ctl[2 * N + v], 1);                       // state iteration of this substep
+  atomicAdd(&w.ctl[4 * N + v], 1);                       // state iterations, total
+  atomicAdd(&w.ctl[5 * N + v], dnewton);                 // Newton iterations, total
   return dnewton;
 }
 
@@ -247,23 +261,21 @@ constitutive_begin_kernel(const __grid_constant__ PhaseConst<NS> pc, const __gri
 }
 
 // one state iteration of every listed voxel: integrateStress (integrateStateFPI:626-629).
-// MINB: resident blocks per SM that the register allocation is bounded for (the variants the
-// autotuner chooses from, stress_variant_blocks); three up to 24 systems by default (168 registers,
-// a few spilled; 67 KB of shared memory per block at 24 systems): measured 5 % faster at 256^3 than
-// two blocks without spills
-template <int NS, int MINB>
-__global__ void __launch_bounds__(pass_threads<NS>(), MINB)
+// MINB: see StressShape (the variants the autotuner chooses from, stress_variant_blocks).
+template <int NS, bool SCHMID, int MINB>
+__global__ void __launch_bounds__(StressShape<NS, SCHMID, MINB>::threads, StressShape<NS, SCHMID, MINB>::blocks)
 constitutive_stress_kernel(const __grid_constant__ PhaseConst<NS> pc, const __grid_constant__ Numerics nm,
                            const __grid_constant__ Fields f, const __grid_constant__ PassWork w, double dt,
                            const int* __restrict__ list_in, int64_t n_in) {
+  using Shape = StressShape<NS, SCHMID, MINB>;
   extern __shared__ double2 smem2[];
-  SysConst* sc = reinterpret_cast<SysConst*>(smem2);
+  auto* sc = reinterpret_cast<StressConst<SCHMID>*>(smem2);
   double* xs = reinterpret_cast<double*>(sc + NS) + threadIdx.x;
-  stage_sys_const<NS>(pc, sc);
+  stage_sys_const<NS>(stress_const(pc, sc), sc);
   __syncthreads();
-  const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t idx = int64_t(blockIdx.x) * Shape::threads + threadIdx.x;
   const bool active = idx < n_in;
-  const int dnewton = active ? stress_voxel<NS>(pc, sc, xs, nm, f, w, list_in[idx], dt) : 0;
+  const int dnewton = active ? stress_voxel<NS, Shape>(pc, sc, xs, nm, f, w, list_in[idx], dt) : 0;
   count_iterations(f.counters, active ? 1 : 0, dnewton);
 }
 
@@ -321,18 +333,19 @@ constitutive_begin_batch_kernel(const __grid_constant__ PhaseConst<NS> pc, const
   append(list_out, count_out, keep, g);
 }
 
-template <int NS>
-__global__ void __launch_bounds__(pass_threads<NS>(), NS > 24 ? 1 : 3)
+template <int NS, bool SCHMID>
+__global__ void __launch_bounds__(StressShape<NS, SCHMID, 3>::threads, StressShape<NS, SCHMID, 3>::blocks)
 constitutive_stress_batch_kernel(const __grid_constant__ PhaseConst<NS> pc, const __grid_constant__ Numerics nm,
                                  const __grid_constant__ BatchTables t, const int* __restrict__ list_in,
                                  const int* __restrict__ count_in) {
+  using Shape = StressShape<NS, SCHMID, 3>;
   const int64_t n_in = *count_in;
   const int64_t first = int64_t(blockIdx.x) * blockDim.x;
   if (first >= n_in) return;
   extern __shared__ double2 smem2[];
-  SysConst* sc = reinterpret_cast<SysConst*>(smem2);
+  auto* sc = reinterpret_cast<StressConst<SCHMID>*>(smem2);
   double* xs = reinterpret_cast<double*>(sc + NS) + threadIdx.x;
-  stage_sys_const<NS>(pc, sc);
+  stage_sys_const<NS>(stress_const(pc, sc), sc);
   __syncthreads();
   for (int64_t base = first; base < n_in; base += int64_t(gridDim.x) * blockDim.x) {
     const int64_t idx = base + threadIdx.x;
@@ -340,7 +353,7 @@ constitutive_stress_batch_kernel(const __grid_constant__ PhaseConst<NS> pc, cons
     if (idx < n_in) {
       const int64_t g = list_in[idx];
       r = t.ctx_of[g];
-      dnewton = stress_voxel<NS>(pc, sc, xs, nm, t.f[r], t.w[r], g - t.off[r], t.dt[r]);
+      dnewton = stress_voxel<NS, Shape>(pc, sc, xs, nm, t.f[r], t.w[r], g - t.off[r], t.dt[r]);
     }
     count_iterations_batch(t.f, r, r >= 0 ? 1 : 0, dnewton);
   }
@@ -423,14 +436,22 @@ int stress_variant_blocks(int ns, int variant) {
 }
 
 namespace {
+template <int NS, bool SCHMID, int MINB>
+cudaError_t launch_stress_as(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f, const PassWork& w, double dt,
+                             const int* list_in, int64_t n_in, cudaStream_t s) {
+  using Shape = StressShape<NS, SCHMID, MINB>;
+  cudaError_t e = cudaFuncSetAttribute(constitutive_stress_kernel<NS, SCHMID, MINB>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(Shape::smem));
+  if (e != cudaSuccess) return e;
+  const int nb = int((n_in + Shape::threads - 1) / Shape::threads);
+  constitutive_stress_kernel<NS, SCHMID, MINB><<<nb, Shape::threads, Shape::smem, s>>>(pc, nm, f, w, dt, list_in, n_in);
+  return cudaGetLastError();
+}
 template <int NS, int MINB>
 cudaError_t launch_stress(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f, const PassWork& w, double dt,
-                          const int* list_in, int64_t n_in, int nb, size_t smem, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(constitutive_stress_kernel<NS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(smem));
-  if (e != cudaSuccess) return e;
-  constitutive_stress_kernel<NS, MINB><<<nb, pass_threads<NS>(), smem, s>>>(pc, nm, f, w, dt, list_in, n_in);
-  return cudaGetLastError();
+                          const int* list_in, int64_t n_in, cudaStream_t s) {
+  return pc.schmid ? launch_stress_as<NS, true, MINB>(pc, nm, f, w, dt, list_in, n_in, s)
+                   : launch_stress_as<NS, false, MINB>(pc, nm, f, w, dt, list_in, n_in, s);
 }
 }  // namespace
 
@@ -438,19 +459,18 @@ template <int NS>
 cudaError_t launch_constitutive_pass(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f,
                                      const PassWork& w, double dt, const int* list_in, int64_t n_in, cudaStream_t s,
                                      int variant) {
-  const size_t smem_s = size_t(NS) * sizeof(SysConst) + size_t(stress_slots<NS>()) * pass_threads<NS>() * sizeof(double);
   const size_t smem_c = (hard_smem_doubles<NS>() + size_t(2 * NS) * pass_threads<NS>()) * sizeof(double);
   cudaError_t e = cudaFuncSetAttribute(constitutive_control_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        int(smem_c));
   if (e != cudaSuccess) return e;
   const int nb = int((n_in + pass_threads<NS>() - 1) / pass_threads<NS>());
   if constexpr (NS > 24) {
-    e = launch_stress<NS, 1>(pc, nm, f, w, dt, list_in, n_in, nb, smem_s, s);
+    e = launch_stress<NS, 1>(pc, nm, f, w, dt, list_in, n_in, s);
   } else {
     switch (stress_variant_blocks(NS, variant)) {
-      case 2: e = launch_stress<NS, 2>(pc, nm, f, w, dt, list_in, n_in, nb, smem_s, s); break;
-      case 4: e = launch_stress<NS, 4>(pc, nm, f, w, dt, list_in, n_in, nb, smem_s, s); break;
-      default: e = launch_stress<NS, 3>(pc, nm, f, w, dt, list_in, n_in, nb, smem_s, s); break;
+      case 2: e = launch_stress<NS, 2>(pc, nm, f, w, dt, list_in, n_in, s); break;
+      case 4: e = launch_stress<NS, 4>(pc, nm, f, w, dt, list_in, n_in, s); break;
+      default: e = launch_stress<NS, 3>(pc, nm, f, w, dt, list_in, n_in, s); break;
     }
   }
   if (e != cudaSuccess) return e;
@@ -459,12 +479,10 @@ cudaError_t launch_constitutive_pass(const PhaseConst<NS>& pc, const Numerics& n
 }
 
 namespace {
-template <int NS>
-int resident_blocks(const void* fn, size_t smem, int nsm, int64_t n_items) {
+int resident_blocks(const void* fn, int threads, size_t smem, int nsm, int64_t n_items) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, pass_threads<NS>(), smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  const int64_t need = (n_items + pass_threads<NS>() - 1) / pass_threads<NS>();
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+  const int64_t need = (n_items + threads - 1) / threads;
   return int(std::max<int64_t>(1, std::min<int64_t>(int64_t(per_sm) * nsm, need)));
 }
 }  // namespace
@@ -472,16 +490,17 @@ int resident_blocks(const void* fn, size_t smem, int nsm, int64_t n_items) {
 // One constitutive evaluation of every active context of a batch as a CUDA graph: prologue, begin
 // kernel (list A), then a while node whose body runs two passes (A -> B, B -> A) and whose
 // condition is set on the device after each pass from the next list's entry count.
-template <int NS>
-cudaError_t build_batch_pass_graph(const PhaseConst<NS>& pc, const Numerics& nm, const BatchTables& t,
-                                   const BatchPassBuffers& b, int nsm, cudaStream_t s, cudaGraph_t* out) {
+template <int NS, bool SCHMID>
+static cudaError_t build_batch_pass_graph_as(const PhaseConst<NS>& pc, const Numerics& nm, const BatchTables& t,
+                                             const BatchPassBuffers& b, int nsm, cudaStream_t s, cudaGraph_t* out) {
   const size_t smem_b = (hard_smem_doubles<NS>() + size_t(2 * NS) * pass_threads<NS>()) * sizeof(double);
-  const size_t smem_s = size_t(NS) * sizeof(SysConst) + size_t(stress_slots<NS>()) * pass_threads<NS>() * sizeof(double);
+  using Shape = StressShape<NS, SCHMID, 3>;
+  const size_t smem_s = Shape::smem;
   const size_t smem_c = smem_b;
   cudaError_t e = cudaFuncSetAttribute(constitutive_begin_batch_kernel<NS>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_b));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(constitutive_stress_batch_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(constitutive_stress_batch_kernel<NS, SCHMID>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              int(smem_s));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(constitutive_control_batch_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -489,10 +508,10 @@ cudaError_t build_batch_pass_graph(const PhaseConst<NS>& pc, const Numerics& nm,
   if (e != cudaSuccess) return e;
   if (t.n_items <= 0 || t.n_items > INT32_MAX) return cudaErrorInvalidValue;
   const int nb_begin = int((t.n_items + pass_threads<NS>() - 1) / pass_threads<NS>());
-  const int nb_s = resident_blocks<NS>(reinterpret_cast<const void*>(constitutive_stress_batch_kernel<NS>), smem_s, nsm,
-                                       t.n_items);
-  const int nb_c = resident_blocks<NS>(reinterpret_cast<const void*>(constitutive_control_batch_kernel<NS>), smem_c,
-                                       nsm, t.n_items);
+  const int nb_s = resident_blocks(reinterpret_cast<const void*>(constitutive_stress_batch_kernel<NS, SCHMID>),
+                                   Shape::threads, smem_s, nsm, t.n_items);
+  const int nb_c = resident_blocks(reinterpret_cast<const void*>(constitutive_control_batch_kernel<NS>), pass_threads<NS>(),
+                                   smem_c, nsm, t.n_items);
   cudaGraph_t g = nullptr;
   if ((e = cudaGraphCreate(&g, 0)) != cudaSuccess) return e;
   auto bail = [&](cudaError_t err) {
@@ -534,7 +553,7 @@ cudaError_t build_batch_pass_graph(const PhaseConst<NS>& pc, const Numerics& nm,
     return bail(e);
   for (int p = 0; p < 2; ++p) {
     const int a = p, z = 1 - p;
-    constitutive_stress_batch_kernel<NS><<<nb_s, pass_threads<NS>(), smem_s, s>>>(pc, nm, t, b.list[a], b.count + a);
+    constitutive_stress_batch_kernel<NS, SCHMID><<<nb_s, Shape::threads, smem_s, s>>>(pc, nm, t, b.list[a], b.count + a);
     constitutive_control_batch_kernel<NS><<<nb_c, pass_threads<NS>(), smem_c, s>>>(pc, nm, t, b.list[a], b.count + a,
                                                                                    b.list[z], b.count + z);
     batch_flip_kernel<<<1, 1, 0, s>>>(b.count + a, b.count + z, b.iter, b.max_passes, h);
@@ -543,6 +562,13 @@ cudaError_t build_batch_pass_graph(const PhaseConst<NS>& pc, const Numerics& nm,
   if (e != cudaSuccess) return bail(e);
   *out = g;
   return cudaSuccess;
+}
+
+template <int NS>
+cudaError_t build_batch_pass_graph(const PhaseConst<NS>& pc, const Numerics& nm, const BatchTables& t,
+                                   const BatchPassBuffers& b, int nsm, cudaStream_t s, cudaGraph_t* out) {
+  return pc.schmid ? build_batch_pass_graph_as<NS, true>(pc, nm, t, b, nsm, s, out)
+                   : build_batch_pass_graph_as<NS, false>(pc, nm, t, b, nsm, s, out);
 }
 
 #define DMK_INSTANTIATE(NS)                                                                                         \

@@ -62,12 +62,13 @@ __device__ __forceinline__ void store_ctl(const PassWork& w, int64_t N, int64_t 
 // compile-time constants, so A stays in registers.
 template <int n>
 __device__ __forceinline__ bool qr_solve(double* A, double* b) {
+  bool bad = false;
 #pragma unroll
   for (int k = 0; k < n - 1; ++k) {
     double s2 = 0.0;
 #pragma unroll
     for (int i = k; i < n; ++i) s2 = fma(A[i * n + k], A[i * n + k], s2);
-    if (s2 == 0.0) return true;
+    bad |= s2 == 0.0;
     const double sig = sqrt(s2);
     const double x0 = A[k * n + k];
     const double alpha = x0 >= 0.0 ? -sig : sig;
@@ -94,7 +95,7 @@ __device__ __forceinline__ bool qr_solve(double* A, double* b) {
     }
     A[k * n + k] = alpha;
   }
-  if (A[n * n - 1] == 0.0) return true;
+  bad |= A[n * n - 1] == 0.0;
 #pragma unroll
   for (int i = n - 1; i >= 0; --i) {
     double s = b[i];
@@ -102,51 +103,114 @@ __device__ __forceinline__ bool qr_solve(double* A, double* b) {
     for (int k = i + 1; k < n; ++k) s = fma(-A[i * n + k], b[k], s);
     b[i] = s / A[i * n + i];
   }
+  return bad;
+}
+
+// Threads and shared-memory slots of the stress kernels.  MINB: warps per scheduler that the registers
+// are bounded for (2, 3 or 4: 255, 168 and 128 registers; 48 systems: three blocks of 64 threads).  A
+// thread's slots (stride: the block's threads): 1/xi (NS), the Newton weights (NS; without non-Schmid
+// terms also K, at least 30), A = F Fp0^-1 (9) and, where they fit, the last accepted Lp (9) and the
+// Newton step (9), which stay in local memory otherwise: the L1 that the slots leave is too small for
+// it, so every read of it goes to L2 (measured).  Blocks of 192 threads where those of 128 leave no room for Lp.
+template <int NS, bool SCHMID, int MINB>
+struct StressShape {
+  static constexpr size_t consts = NS * sizeof(StressConst<SCHMID>) + 1024;   // with the system's 1 KB per block
+  static constexpr int base = NS + (SCHMID && NS < 30 ? 30 : NS) + 9;
+  static constexpr bool fits(int slots, int threads, int blocks) {
+    return blocks * (consts + sizeof(double) * slots * threads) <= 228 * 1024;
+  }
+  static constexpr bool wide = NS <= 24 && MINB == 3 && !fits(base + 9, 128, 3) && fits(base + 9, 192, 2);
+  static constexpr int threads = NS > 24 ? 64 : wide ? 192 : 128;
+  static constexpr int blocks = NS > 24 ? 3 : wide ? 2 : MINB;
+  static constexpr bool lo_shared = fits(base + 9, threads, blocks);
+  static constexpr bool dl_shared = fits(base + 18, threads, blocks);
+  static constexpr int slots = base + (lo_shared ? 9 : 0) + (dl_shared ? 9 : 0);
+  static constexpr size_t smem = NS * sizeof(StressConst<SCHMID>) + sizeof(double) * slots * threads;
+};
+
+// nine values of a thread that are read rarely: in its shared-memory slots (stride T) or in local memory
+template <bool SHARED, int T>
+struct Rare9 {
+  double* s;
+  __device__ explicit Rare9(double* p) : s(p) {}
+  __device__ double get(int k) const { return s[k * T]; }
+  __device__ void set(int k, double x) { s[k * T] = x; }
+};
+template <int T>
+struct Rare9<false, T> {
+  volatile double a[9];
+  __device__ explicit Rare9(double*) {}
+  __device__ double get(int k) const { return a[k]; }
+  __device__ void set(int k, double x) { a[k] = x; }
+};
+
+// A = F Fp0^-1 into the thread's slots; true if Fp0 is singular
+template <int T>
+__device__ __forceinline__ bool stress_begin(const double* F, const double* Fp0, double* sA) {
+  double invFp0[9], A[9];
+  if (inv33(Fp0, invFp0)) return true;
+  mm33(F, invFp0, A);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) sA[k * T] = A[k];
   return false;
 }
 
-// integrateStress, phase_mechanical.f90:379-584 (Fi = I, Li = 0).
-// F and Fp0 point at voxel v's planes (stride N); they are read at the start and again
-// for the final Fp / P so that no copy stays in registers through the Newton loop.
-// xs: this thread's shared-memory slots (stride pass_threads<NS>()): 1/xi (NS entries), the
-// Newton weights dt*dgamma (NS), then A (9).  The voxel's planes (stride N) receive |dot_gamma|
-// of the last residual evaluation (adg_g; the state update after a converged integration reads
-// it), the last accepted Lp guess (lo_g) and the Newton step (dl_g): they are written once per
-// Newton iteration and read back rarely (line search, step), so they stay out of the shared
-// memory that bounds the kernel's occupancy.  Lp (in/out) is the warm start and, on success,
-// the result; S, Fp, P and Fe are written only on success.
-template <int NS>
-__device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __restrict__ sc, const Numerics& nm,
-                                const double* Fg, const double* Fp0g, int64_t N, double* xs, double dt, double* Lp,
-                                double* S, double* Fp, double* Pout, double* Feout, int& newton,
-                                double* __restrict__ adg_g, double* __restrict__ lo_g, double* __restrict__ dl_g) {
-  double* const sw = xs + NS * pass_threads<NS>();
-  double* const sA = xs + 2 * NS * pass_threads<NS>();
+// Fp = (Fp0^-1 B)^-1 / det^(1/3); P = F Fp^-1 S Fp^-T = Fe S Fp^-T (phase_mechanical.f90:571-581; Fe =
+// F Fp0^-1 B is the last iterate's); Fp0 is read again, so that nothing of it stays in registers
+// through the Newton loop.  Returns the status of the integration.
+__device__ __forceinline__ int stress_end(const double* Fp0g, int64_t N, const double* B, const double* Fe,
+                                          const double* s6, double* Fp, double* Pout) {
+  double invFpn[9], Fpn[9];
   {
-    double F[9], Fp0[9], invFp0[9], A[9];
+    double Fp0[9], invFp0[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) { F[k] = Fg[k * N]; Fp0[k] = Fp0g[k * N]; }
-    if (inv33(Fp0, invFp0)) return 5;                     // STATUS_FAIL_PHASE_MECHANICAL_STRESS
-    mm33(F, invFp0, A);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) sA[k * pass_threads<NS>()] = A[k];
+    for (int k = 0; k < 9; ++k) Fp0[k] = Fp0g[k * N];
+    inv33(Fp0, invFp0);                                   // invertible: checked on entry
+    mm33(invFp0, B, invFpn);
   }
+  if (inv33(invFpn, Fpn)) return 5;
+  const double cb = 1.0 / cbrt(det33(Fpn));
+  const double Sm[9] = {s6[0], s6[5], s6[4], s6[5], s6[1], s6[3], s6[4], s6[3], s6[2]};
+  double T1[9];
+  mmt33(Sm, invFpn, T1);          // S Fp^-T
+  mm33(Fe, T1, Pout);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) Fp[k] = Fpn[k] * cb;
+  return 0;
+}
 
+// integrateStress, phase_mechanical.f90:379-584 (Fi = I, Li = 0).
+// F, Fp0: the values of voxel v; Fp0g: its Fp0 planes (stride N), read again for the final Fp / P.
+// xs: this thread's shared-memory slots (see StressShape).  adg_g: the voxel's plane of |dot_gamma|
+// (stride N), written in every residual evaluation for the state update after a converged integration.
+// Lp (in/out) is the warm start and, on success, the result; S, Fp and P are written only on success; Fe is
+// the last iterate's.
+template <int NS, class Shape>
+__device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __restrict__ sc, const Numerics& nm,
+                                const double* F, const double* Fp0, const double* Fp0g, int64_t N, double* xs, double dt,
+                                double* Lp, double* S, double* Fp, double* Pout, double* Fe, int& newton,
+                                double* __restrict__ adg_g) {
+  constexpr int T = Shape::threads;
+  double* const sw = xs + NS * T;
+  double* const sA = xs + (Shape::base - 9) * T;
+  if (stress_begin<T>(F, Fp0, sA)) return 5;        // STATUS_FAIL_PHASE_MECHANICAL_STRESS
+
+  Rare9<Shape::lo_shared, T> lo(xs + Shape::base * T);
+  Rare9<Shape::dl_shared, T> dl(xs + (Shape::base + 9) * T);
   double Lg[9], B[9], s6[6];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) { Lg[k] = Lp[k]; lo_g[k * N] = Lp[k]; dl_g[k * N] = 0.0; }
+  for (int k = 0; k < 9; ++k) { Lg[k] = Lp[k]; lo.set(k, Lp[k]); dl.set(k, 0.0); }
   double step = 1.0, res_old = 1.7976931348623157e308;
   int jaco = 0;
   for (int it = 1;; ++it) {
     if (it > nm.N_iter_Lp_max) return 6;                  // STATUS_FAIL_PHASE_MECHANICAL_STRESS_LP_MAXIT
     ++newton;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) B[k] = ((k % 4 == 0) ? 1.0 : 0.0) - dt * Lg[k];
-    double Fe[9];
+    for (int k = 0; k < 9; ++k) B[k] = fma(-dt, Lg[k], (k % 4 == 0) ? 1.0 : 0.0);
     {
       double A[9];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) A[k] = sA[k * pass_threads<NS>()];
+      for (int k = 0; k < 9; ++k) A[k] = sA[k * T];
       mm33(A, B, Fe);
     }
     hooke_S<NS>(pc, Fe, s6);
@@ -160,11 +224,11 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
       double2 p[6];
 #pragma unroll
       for (int t = 0; t < 6; ++t) p[t] = c.p6[t];
-      const double tp = s6[0] * p[0].x + s6[1] * p[1].x + s6[2] * p[2].x + s6[3] * p[3].x + s6[4] * p[4].x + s6[5] * p[5].x;
-      const double tn = s6[0] * p[0].y + s6[1] * p[1].y + s6[2] * p[2].y + s6[3] * p[3].y + s6[4] * p[4].y + s6[5] * p[5].y;
+      const double tp = fma(s6[5], p[5].x, fma(s6[4], p[4].x, fma(s6[3], p[3].x, dot3(s6[0], p[0].x, s6[1], p[1].x, s6[2], p[2].x))));
+      const double tn = fma(s6[5], p[5].y, fma(s6[4], p[4].y, fma(s6[3], p[3].y, dot3(s6[0], p[0].y, s6[1], p[1].y, s6[2], p[2].y))));
       const bool pos = tp > tn;
       const double tmax = pos ? tp : tn;
-      const double ixs = xs[s * pass_threads<NS>()];
+      const double ixs = xs[s * T];
       const double r = tmax * ixs;
       const double2 kin = c.kin;
       const int ni = c.n_int;
@@ -181,7 +245,7 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
       if (!(fabs(g) > TINY10)) dg = 0.0;
       // P_nS sense of the derivative follows the sign of dot_gamma (phenopowerlaw.f90:327)
       if (!(g > 0.0)) neg |= SenseMask<NS>(1) << s;
-      sw[s * pass_threads<NS>()] = dt * dg;
+      sw[s * T] = dt * dg;
       adg_g[s * N] = fabs(g);
       double2 P[5];
 #pragma unroll
@@ -200,14 +264,15 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
     if (nR < res_old) {
       res_old = nR;
 #pragma unroll
-      for (int k = 0; k < 9; ++k) lo_g[k * N] = Lg[k];
+      for (int k = 0; k < 9; ++k) lo.set(k, Lg[k]);
       step = 1.0;
     } else {
       step = nm.r_linesearch_Lp * step;
 #pragma unroll
-      for (int k = 0; k < 9; ++k) Lg[k] = fma(dl_g[k * N], step, lo_g[k * N]);
+      for (int k = 0; k < 9; ++k) Lg[k] = fma(dl.get(k), step, lo.get(k));
       continue;
     }
+    double X[9];
     if (jaco % nm.f_update_jacobi_Lp == 0) {
       ++jaco;
       // Newton step J dLp = -R with J = I + K, K[kl][pb] = (M H^(kl))(p,b), M = A^T Fe,
@@ -221,7 +286,7 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
       {
         double A[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) A[k] = sA[k * pass_threads<NS>()];
+        for (int k = 0; k < 9; ++k) A[k] = sA[k * T];
         mtm33(A, Fe, M);                                  // M = A^T Fe, M[p + 3q] = M(p,q)
       }
       double C6[36];
@@ -230,7 +295,7 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
 #pragma unroll 2
       for (int s = 0; s < NS; ++s) {
         const SysConst& c = sc[s];
-        const double ws = sw[s * pass_threads<NS>()];
+        const double ws = sw[s * T];
         const bool ng = (neg >> s) & 1u;
         double q[6];
 #pragma unroll
@@ -241,11 +306,11 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
         const double2 dn0 = c.dn[0], dn1 = c.dn[1], dn2 = c.dn[2];
         const double d0 = dn0.x, d1 = dn0.y, d2 = dn1.x, n0 = dn1.y, n1 = dn2.x, n2 = dn2.y;
         // u = M^T d
-        const double u0 = M[0] * d0 + M[1] * d1 + M[2] * d2;
-        const double u1 = M[3] * d0 + M[4] * d1 + M[5] * d2;
-        const double u2 = M[6] * d0 + M[7] * d1 + M[8] * d2;
-        const double a6[6] = {ws * (u0 * n0), ws * (u1 * n1), ws * (u2 * n2), ws * (u1 * n2 + u2 * n1),
-                              ws * (u0 * n2 + u2 * n0), ws * (u0 * n1 + u1 * n0)};
+        const double u0 = dot3(M[0], d0, M[1], d1, M[2], d2);
+        const double u1 = dot3(M[3], d0, M[4], d1, M[5], d2);
+        const double u2 = dot3(M[6], d0, M[7], d1, M[8], d2);
+        const double a6[6] = {ws * (u0 * n0), ws * (u1 * n1), ws * (u2 * n2), ws * fma(u1, n2, u2 * n1),
+                              ws * fma(u0, n2, u2 * n0), ws * fma(u0, n1, u1 * n0)};
 #pragma unroll
         for (int i = 0; i < 6; ++i)
 #pragma unroll
@@ -260,7 +325,6 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
         y6[3] = G[7] + G[5]; y6[4] = G[6] + G[2]; y6[5] = G[3] + G[1];
       }
       if (qr_solve<6>(C6, y6)) return 8;                 // singular: STATUS_FAIL_PHASE_MECHANICAL_STRESS_LP_DGESV
-      double X[9];
 #pragma unroll
       for (int k = 0; k < 9; ++k) X[k] = -R[k];
 #pragma unroll 2
@@ -273,7 +337,7 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
           const double2 qq = c.q6[t];
           cq = fma(ng ? qq.y : qq.x, y6[t], cq);
         }
-        cq *= sw[s * pass_threads<NS>()];
+        cq *= sw[s * T];
         double2 P[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) P[k] = c.P[k];
@@ -282,30 +346,225 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
         for (int k = 0; k < 9; ++k) X[k] = fma(cq, Ps[k], X[k]);
       }
 #pragma unroll
-      for (int k = 0; k < 9; ++k) dl_g[k * N] = X[k];
+      for (int k = 0; k < 9; ++k) dl.set(k, X[k]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) X[k] = dl.get(k);
     }
 #pragma unroll
-    for (int k = 0; k < 9; ++k) Lg[k] = fma(dl_g[k * N], step, Lg[k]);
+    for (int k = 0; k < 9; ++k) Lg[k] = fma(X[k], step, Lg[k]);
   }
-  // Fp = (Fp0^-1 B)^-1 / det^(1/3); P = F Fp^-1 S Fp^-T; Fe = F Fp^-1  (:571-581)
-  double F[9], invFpn[9], Fpn[9];
-  {
-    double Fp0[9], invFp0[9];
+  if (stress_end(Fp0g, N, B, Fe, s6, Fp, Pout)) return 5;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) { F[k] = Fg[k * N]; Fp0[k] = Fp0g[k * N]; }
-    inv33(Fp0, invFp0);                                   // invertible: checked on entry
-    mm33(invFp0, B, invFpn);
+  for (int k = 0; k < 9; ++k) Lp[k] = Lg[k];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) S[k] = s6[k];
+  return 0;
+}
+
+// The same for a phase without non-Schmid terms and cubic elasticity (every phase of this path has the
+// latter).  Both senses of a system then share P_s, so tau = S : P_s with the sign of dot_gamma taken
+// from it, and C : P_s is traceless.  With the coordinates (u, v) of P_s (SchmidConst) and
+//   zeta(Y) = (CY11 - CY33, CY22 - CY33, 2 CY23, 2 CY13, 2 CY12), CY = C : sym(Y),
+// the resolved shear of E is u . zeta(E) and the rank-6 system of the general form closes in five unknowns:
+//   K_k = sum_s w_s P_s u_s,k,   z + sum_k zeta(M^T K_k) z_k = zeta(M^T R),   dLp = sum_k K_k z_k - R.
+// The u-u part of K is symmetric, so a system adds 15 + 15 products to it instead of 36 to C6, and dLp needs
+// no second pass over the systems.  What bounds the kernel is the FP64 instructions of this function and
+// the latency of their chains at twelve warps per SM (more warps have no registers), then every memory
+// round trip that they cannot hide: all of a voxel's loads are issued at once (stress_voxel), and nothing
+// of the loop lives in memory (spills and planes of the Newton step went to L2: the slots leave little of
+// L1).  Stress kernels of one increment, general form with its loads one after the other -> this: 24
+// systems at 128^3 147 -> 94 ms, 48 systems at 40^3 17.5 -> 9.7 ms, 12 systems at 64^3 9.5 -> 6.8 ms;
+// FP64 pipe 35 -> 51 % busy, long-scoreboard stalls per issue 2.0 -> 0.45.
+template <int NS, class Shape>
+__device__ int integrate_stress(const PhaseConst<NS>& pc, const SchmidConst* __restrict__ sc, const Numerics& nm,
+                                const double* F, const double* Fp0, const double* Fp0g, int64_t N, double* xs, double dt,
+                                double* Lp, double* S, double* Fp, double* Pout, double* Fe, int& newton,
+                                double* __restrict__ adg_g) {
+  constexpr int T = Shape::threads;
+  double* const sw = xs + NS * T;                         // weights, then K (15 + 15 products)
+  double* const sA = xs + (Shape::base - 9) * T;
+  if (stress_begin<T>(F, Fp0, sA)) return 5;        // STATUS_FAIL_PHASE_MECHANICAL_STRESS
+  const double c1 = pc.C66[0][0] - pc.C66[0][1], c4 = pc.C66[3][3];   // C11 - C12, 2 C44
+
+  Rare9<Shape::lo_shared, T> lo(xs + Shape::base * T);
+  Rare9<Shape::dl_shared, T> dl(xs + (Shape::base + 9) * T);
+  double Lg[9], B[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) { Lg[k] = Lp[k]; lo.set(k, Lp[k]); dl.set(k, 0.0); }
+  double step = 1.0, res_old = 1.7976931348623157e308;
+  int jaco = 0;
+  for (int it = 1;; ++it) {
+    if (it > nm.N_iter_Lp_max) return 6;                  // STATUS_FAIL_PHASE_MECHANICAL_STRESS_LP_MAXIT
+    ++newton;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) B[k] = fma(-dt, Lg[k], (k % 4 == 0) ? 1.0 : 0.0);
+    {
+      double A[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) A[k] = sA[k * T];
+      mm33(A, B, Fe);
+    }
+    double z[5];                                          // zeta(E), E = (Fe^T Fe - I)/2
+    {
+      const double f33 = dot3(Fe[6], Fe[6], Fe[7], Fe[7], Fe[8], Fe[8]);
+      z[0] = (0.5 * c1) * (dot3(Fe[0], Fe[0], Fe[1], Fe[1], Fe[2], Fe[2]) - f33);
+      z[1] = (0.5 * c1) * (dot3(Fe[3], Fe[3], Fe[4], Fe[4], Fe[5], Fe[5]) - f33);
+      z[2] = c4 * dot3(Fe[3], Fe[6], Fe[4], Fe[7], Fe[5], Fe[8]);
+      z[3] = c4 * dot3(Fe[0], Fe[6], Fe[1], Fe[7], Fe[2], Fe[8]);
+      z[4] = c4 * dot3(Fe[0], Fe[3], Fe[1], Fe[4], Fe[2], Fe[5]);
+    }
+    // Lp_c = sum_s dot_gamma_s P_s and the weights of its derivative
+    double R[9];
+    {
+      double l[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 2
+      for (int s = 0; s < NS; ++s) {
+        const double2 u01 = sc[s].u01, u23 = sc[s].u23, u4v0 = sc[s].u4v0, v12 = sc[s].v12, kin = sc[s].kin;
+        const double tau = fma(u01.x, z[0], u01.y * z[1]) + fma(u23.x, z[2], fma(u23.y, z[3], u4v0.x * z[4]));
+        const double ta = fabs(tau);
+        const double ixs = xs[s * T];
+        const double r = ta * ixs;
+        const int ni = sc[s].n_int;
+        double g, dg;                                      // |dot_gamma| and its derivative
+        if (ni >= 1) {
+          const double rn1 = powi_fixed<6>(r, ni - 1);
+          g = (kin.x * rn1) * r;
+          dg = (kin.x * kin.y) * rn1 * ixs;
+        } else {
+          g = kin.x * pow(r, kin.y);
+          dg = g * kin.y / ta;
+        }
+        if (!(g > TINY10)) dg = 0.0;
+        sw[s * T] = dt * dg;
+        adg_g[s * N] = g;
+        g = copysign(g, tau);
+        l[0] = fma(g, u01.x, l[0]);
+        l[1] = fma(g, u01.y, l[1]);
+        l[2] = fma(g, u23.x, l[2]);
+        l[3] = fma(g, u23.y, l[3]);
+        l[4] = fma(g, u4v0.x, l[4]);
+        l[5] = fma(g, u4v0.y, l[5]);
+        l[6] = fma(g, v12.x, l[6]);
+        l[7] = fma(g, v12.y, l[7]);
+      }
+      const double Lc[9] = {l[0], l[4] - l[7], l[3] - l[6], l[4] + l[7], l[1], l[2] - l[5], l[3] + l[6], l[2] + l[5],
+                            -(l[0] + l[1])};
+#pragma unroll
+      for (int k = 0; k < 9; ++k) R[k] = Lg[k] - Lc[k];
+      const double nR = norm9(R);
+      const double atol = fmax(nm.eps_rel_Lp * fmax(norm9(Lg), norm9(Lc)), nm.eps_abs_Lp);
+      if (isnan(nR)) return 7;                            // STATUS_FAIL_PHASE_MECHANICAL_STRESS_LP_NAN
+      if (nR < atol) break;
+      if (nR < res_old) {
+        res_old = nR;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) lo.set(k, Lg[k]);
+        step = 1.0;
+      } else {
+        step = nm.r_linesearch_Lp * step;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) Lg[k] = fma(dl.get(k), step, lo.get(k));
+        continue;
+      }
+    }
+    double X[9];
+    if (jaco % nm.f_update_jacobi_Lp == 0) {
+      ++jaco;
+      // K: columns k of u-u products (symmetric: 15) and v-u products (15)
+      double Ku[15], Kv[15];
+#pragma unroll
+      for (int i = 0; i < 15; ++i) Ku[i] = Kv[i] = 0.0;
+#pragma unroll 1
+      for (int s = 0; s < NS; ++s) {
+        const double2 u01 = sc[s].u01, u23 = sc[s].u23, u4v0 = sc[s].u4v0, v12 = sc[s].v12;
+        const double u[5] = {u01.x, u01.y, u23.x, u23.y, u4v0.x};
+        const double v[3] = {u4v0.y, v12.x, v12.y};
+        const double w = sw[s * T];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+          const double wu = w * u[k];
+#pragma unroll
+          for (int i = 0; i <= k; ++i) Ku[k * (k + 1) / 2 + i] = fma(wu, u[i], Ku[k * (k + 1) / 2 + i]);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) Kv[3 * k + i] = fma(wu, v[i], Kv[3 * k + i]);
+        }
+      }
+      double M[9];
+      {
+        double A[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) A[k] = sA[k * T];
+        mtm33(A, Fe, M);                                  // M = A^T Fe
+      }
+      // zeta(M^T Y) but for the factors c1, c1, c4, c4, c4
+      auto zeta = [&](const double* Y, double* o) {
+        const double g33 = dot3(M[6], Y[6], M[7], Y[7], M[8], Y[8]);
+        o[0] = dot3(M[0], Y[0], M[1], Y[1], M[2], Y[2]) - g33;
+        o[1] = dot3(M[3], Y[3], M[4], Y[4], M[5], Y[5]) - g33;
+        o[2] = dot3(M[3], Y[6], M[4], Y[7], M[5], Y[8]) + dot3(M[6], Y[3], M[7], Y[4], M[8], Y[5]);
+        o[3] = dot3(M[0], Y[6], M[1], Y[7], M[2], Y[8]) + dot3(M[6], Y[0], M[7], Y[1], M[8], Y[2]);
+        o[4] = dot3(M[0], Y[3], M[1], Y[4], M[2], Y[5]) + dot3(M[3], Y[0], M[4], Y[1], M[5], Y[2]);
+      };
+      // K goes to the slots of the weights, which are spent, so that J and the factorisation have the registers
+#pragma unroll
+      for (int i = 0; i < 15; ++i) {
+        sw[i * T] = Ku[i];
+        sw[(15 + i) * T] = Kv[i];
+      }
+      asm volatile("" ::: "memory");                      // keep K there: no forwarding from the registers
+      auto ku = [&](int k, int i) { return sw[(i <= k ? k * (k + 1) / 2 + i : i * (i + 1) / 2 + k) * T]; };
+      auto kv = [&](int k, int i) { return sw[(15 + 3 * k + i) * T]; };
+      double y[5];
+      zeta(R, y);
+#pragma unroll
+      for (int i = 0; i < 5; ++i) y[i] *= i < 2 ? c1 : c4;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) dl.set(k, R[k]);
+      asm volatile("" ::: "memory");                      // and R
+      double J[25];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        double u[5], v[3];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) u[i] = ku(k, i);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) v[i] = kv(k, i);
+        const double Y[9] = {u[0], u[4] - v[2], u[3] - v[1], u[4] + v[2], u[1], u[2] - v[0], u[3] + v[1], u[2] + v[0],
+                             -(u[0] + u[1])};
+        double o[5];
+        zeta(Y, o);
+#pragma unroll
+        for (int i = 0; i < 5; ++i) J[5 * i + k] = fma(i < 2 ? c1 : c4, o[i], i == k ? 1.0 : 0.0);
+      }
+      if (qr_solve<5>(J, y)) return 8;                   // singular: STATUS_FAIL_PHASE_MECHANICAL_STRESS_LP_DGESV
+      double d[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+#pragma unroll
+        for (int i = 0; i < 5; ++i) d[i] = fma(ku(k, i), y[k], d[i]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) d[5 + i] = fma(kv(k, i), y[k], d[5 + i]);
+      }
+      const double D[9] = {d[0], d[4] - d[7], d[3] - d[6], d[4] + d[7], d[1], d[2] - d[5], d[3] + d[6], d[2] + d[5],
+                           -(d[0] + d[1])};
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        X[k] = D[k] - dl.get(k);
+        dl.set(k, X[k]);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) X[k] = dl.get(k);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Lg[k] = fma(X[k], step, lo.get(k));
   }
-  if (inv33(invFpn, Fpn)) return 5;
-  const double cb = 1.0 / cbrt(det33(Fpn));
-  double FiF[9];
-  mm33(F, invFpn, FiF);
-  const double Sm[9] = {s6[0], s6[5], s6[4], s6[5], s6[1], s6[3], s6[4], s6[3], s6[2]};
-  double T1[9], T2[9];
-  mmt33(Sm, invFpn, T1);          // S Fp^-T
-  mm33(FiF, T1, T2);
+  double s6[6];
+  hooke_S<NS>(pc, Fe, s6);
+  if (stress_end(Fp0g, N, B, Fe, s6, Fp, Pout)) return 5;
 #pragma unroll
-  for (int k = 0; k < 9; ++k) { Pout[k] = T2[k]; Feout[k] = FiF[k]; Fp[k] = Fpn[k] * cb; Lp[k] = Lg[k]; }
+  for (int k = 0; k < 9; ++k) Lp[k] = Lg[k];
 #pragma unroll
   for (int k = 0; k < 6; ++k) S[k] = s6[k];
   return 0;
@@ -323,11 +582,6 @@ template <int NS>
 __device__ __forceinline__ void stage_hardening(const PhaseConst<NS>& pc, double* hs) {
   for (int i = threadIdx.x; i < NS * NS; i += blockDim.x) hs[i] = pc.hmat[i];
 }
-
-// Slots of the stress kernel (stride pass_threads<NS>()): 1/xi [0, NS), Newton weights
-// [NS, 2NS), A = F Fp0^-1 [2NS, 2NS + 9).
-template <int NS>
-__host__ __device__ constexpr int stress_slots() { return 2 * NS + 9; }
 
 // phenopowerlaw_dotState (Fi = I => Mp = S; no twins => sumF = 0) at the stored
 // stress and state of voxel v, written to this thread's slots: xi rates first, then
@@ -504,9 +758,9 @@ __device__ void advance(const PhaseConst<NS>& pc, const double* __restrict__ hs,
 #pragma unroll 12
         for (int i = 0; i < NST; ++i) {
           const double l1 = L1[i * N];
-          const double d = xs[i * pass_threads<NS>()] * zeta + l1 * (1.0 - zeta);
+          const double d = fma(xs[i * pass_threads<NS>()], zeta, l1 * (1.0 - zeta));
           const double st = f.state[i * N + v];
-          const double r = st - st0[i * N + v] - d * dts;
+          const double r = fma(-d, dts, st - st0[i * N + v]);
           const double stn = st - r;
           f.state[i * N + v] = stn;
           L2[i * N] = d;

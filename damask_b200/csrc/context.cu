@@ -76,6 +76,7 @@ struct dmk_ctx {
   PhaseConst<48>* pc48 = nullptr;
   double* hmat = nullptr;        // slip-slip hardening matrix (NS x NS), read by the pass kernels
   SysConst* sysc = nullptr;      // per-system constants of the Newton loop (NS entries)
+  SchmidConst* schmidc = nullptr;   // the same for a phase without non-Schmid terms (else null)
   Numerics nm;
   Numerics2 nm2;
   GammaConst gc;
@@ -201,14 +202,12 @@ PassWork pass_work(dmk_ctx* c, int half, int out) {
   w.adg = w.D + 2 * NST * N;
   w.dot0 = c->dot0;
   w.sub = w.adg + int64_t(c->NS) * N;
-  w.lo = w.sub + 2 * N;
-  w.dl = w.lo + 9 * N;
   w.ctl = c->pctl;
   w.list_out = c->plist[half][out];
   w.count_out = c->pcount + 2 * half + out;
   return w;
 }
-size_t pass_work_doubles(int64_t N, int NS) { return size_t(N) * size_t(36 + 7 * NS + 2 + 18); }
+size_t pass_work_doubles(int64_t N, int NS) { return size_t(N) * size_t(36 + 7 * NS + 2); }
 
 template <int NS>
 int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, double dt, int apply) {
@@ -1080,24 +1079,35 @@ int dmk_mech_init(dmk_ctx** out, const int cells[3], const double geomSize[3], c
   }
   {
     // per-system constants of the Newton loop, staged into shared memory by the pass kernels
-    std::vector<SysConst> sys(c->NS);
-    for (int i = 0; i < c->NS; ++i) {
-      switch (c->NS) {
-        case 12: sys[i] = make_sys_const<12>(*c->pc12, i); break;
-        case 18: sys[i] = make_sys_const<18>(*c->pc18, i); break;
-        case 24: sys[i] = make_sys_const<24>(*c->pc24, i); break;
-        case 48: sys[i] = make_sys_const<48>(*c->pc48, i); break;
+    auto upload = [&](auto& pc) -> int {
+      std::vector<SysConst> sys(c->NS);
+      std::vector<SchmidConst> schmid(c->NS);
+      for (int i = 0; i < c->NS; ++i) {
+        sys[i] = make_sys_const(pc, i);
+        schmid[i] = make_schmid_const(pc, i);
       }
-    }
-    if (cudaMalloc(&c->sysc, sizeof(SysConst) * c->NS) != cudaSuccess ||
-        cudaMemcpy(c->sysc, sys.data(), sizeof(SysConst) * c->NS, cudaMemcpyHostToDevice) != cudaSuccess)
-      return bail(fail(DMK_ERR_CUDA, "copy of the per-system constants failed"));
+      // without non-Schmid terms both senses of every system are +-P_s, and the stress kernels take
+      // the five-unknown form
+      bool plain = true;
+      for (int i = 0; i < c->NS; ++i)
+        for (int k = 0; k < 9; ++k) plain = plain && pc.PnS[0][i][k] == pc.P[i][k] && pc.PnS[1][i][k] == -pc.P[i][k];
+      if (cudaMalloc(&c->sysc, sizeof(SysConst) * c->NS) != cudaSuccess ||
+          cudaMemcpy(c->sysc, sys.data(), sizeof(SysConst) * c->NS, cudaMemcpyHostToDevice) != cudaSuccess)
+        return fail(DMK_ERR_CUDA, "copy of the per-system constants failed");
+      if (plain && (cudaMalloc(&c->schmidc, sizeof(SchmidConst) * c->NS) != cudaSuccess ||
+                    cudaMemcpy(c->schmidc, schmid.data(), sizeof(SchmidConst) * c->NS, cudaMemcpyHostToDevice) != cudaSuccess))
+        return fail(DMK_ERR_CUDA, "copy of the per-system constants failed");
+      pc.sys = c->sysc;
+      pc.schmid = c->schmidc;
+      return 0;
+    };
     switch (c->NS) {
-      case 12: c->pc12->sys = c->sysc; break;
-      case 18: c->pc18->sys = c->sysc; break;
-      case 24: c->pc24->sys = c->sysc; break;
-      case 48: c->pc48->sys = c->sysc; break;
+      case 12: rc = upload(*c->pc12); break;
+      case 18: rc = upload(*c->pc18); break;
+      case 24: rc = upload(*c->pc24); break;
+      case 48: rc = upload(*c->pc48); break;
     }
+    if (rc) return bail(rc);
   }
 
   const int NST = 2 * c->NS;
@@ -1826,6 +1836,7 @@ void dmk_destroy(dmk_ctx* c) {
   delete c->pc48;
   if (c->hmat) cudaFree(c->hmat);
   if (c->sysc) cudaFree(c->sysc);
+  if (c->schmidc) cudaFree(c->schmidc);
   delete c;
 }
 
@@ -2302,6 +2313,7 @@ bool same_phase_const(const dmk_ctx* a, const dmk_ctx* b) {
   auto y = std::make_unique<PhaseConst<NS>>(*phase_const_of<NS>(b));
   x->hmat = y->hmat = nullptr;
   x->sys = y->sys = nullptr;
+  x->schmid = y->schmid = nullptr;
   return std::memcmp(x.get(), y.get(), sizeof(PhaseConst<NS>)) == 0;
 }
 bool same_phase(const dmk_ctx* a, const dmk_ctx* b) {

@@ -15,6 +15,7 @@ namespace dmk {
 constexpr double TINY10 = 10.0 * 2.2250738585072014e-308;   // dEq0 threshold, prec.f90:131-143
 
 struct SysConst;
+struct SchmidConst;
 
 // Per-phase constants, passed by value as a __grid_constant__ kernel parameter so
 // that every uniform access is served by the constant bank.
@@ -30,6 +31,7 @@ struct PhaseConst {
   double dg0[NS], n[NS], a[NS], h0f[NS], xiinf[NS], ixiinf[NS];
   const double* hmat;      // slip-slip hardening matrix (NS x NS, row = reacting system) in device memory
   const SysConst* sys;     // the per-system constants of the Newton loop (NS entries) in device memory
+  const SchmidConst* schmid;   // the same for a phase without non-Schmid terms (NS entries), else null
   int n_int[NS];           // stress exponent as integer if integral, else -1
   int a_int[NS];           // hardening exponent as integer if integral, else -1
   double atol_xi, atol_gamma;
@@ -87,8 +89,6 @@ struct PassWork {
   double* adg;     // NS: |dot_gamma| at the stress of the last converged integrateStress
   double* dot0;    // 2 NS: dotState at the increment-start stress and state (S0, state0)
   double* sub;     // 2: stepFrac (subFrac), step (subStep)
-  double* lo;      // 9: the last accepted Lp guess of the current integrateStress
-  double* dl;      // 9: its Newton step
   int* ctl;        // 6: phase, status, state iteration, substeps, state iterations total, Newton total
   int* list_out;   // voxels that continue into the next pass
   int* count_out;  // number of entries appended to list_out
@@ -102,13 +102,19 @@ struct VoxelCtl {
 };
 
 // ------------------------------------------------------------- 3x3 helpers
+// Sums of products are written as explicit fma chains, here and in the passes: which product of a
+// sum is fused is then not the compiler's choice in each kernel, and the kernels of one context, of a
+// batch and of every register bound round alike.
+__device__ __forceinline__ double dot3(double a0, double b0, double a1, double b1, double a2, double b2) {
+  return fma(a2, b2, fma(a0, b0, a1 * b1));
+}
+__device__ __forceinline__ double cross2(double a, double b, double c, double d) { return fma(a, b, -(c * d)); }   // ab - cd
 // Column-major: a[i + 3*j] = A(i,j)
 __device__ __forceinline__ void mm33(const double* A, const double* B, double* C) {
 #pragma unroll
   for (int j = 0; j < 3; ++j)
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-      C[i + 3 * j] = A[i] * B[3 * j] + A[i + 3] * B[1 + 3 * j] + A[i + 6] * B[2 + 3 * j];
+    for (int i = 0; i < 3; ++i) C[i + 3 * j] = dot3(A[i], B[3 * j], A[i + 3], B[1 + 3 * j], A[i + 6], B[2 + 3 * j]);
 }
 // C = A^T B
 __device__ __forceinline__ void mtm33(const double* A, const double* B, double* C) {
@@ -116,32 +122,32 @@ __device__ __forceinline__ void mtm33(const double* A, const double* B, double* 
   for (int j = 0; j < 3; ++j)
 #pragma unroll
     for (int i = 0; i < 3; ++i)
-      C[i + 3 * j] = A[3 * i] * B[3 * j] + A[1 + 3 * i] * B[1 + 3 * j] + A[2 + 3 * i] * B[2 + 3 * j];
+      C[i + 3 * j] = dot3(A[3 * i], B[3 * j], A[1 + 3 * i], B[1 + 3 * j], A[2 + 3 * i], B[2 + 3 * j]);
 }
 // C = A B^T
 __device__ __forceinline__ void mmt33(const double* A, const double* B, double* C) {
 #pragma unroll
   for (int j = 0; j < 3; ++j)
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-      C[i + 3 * j] = A[i] * B[j] + A[i + 3] * B[j + 3] + A[i + 6] * B[j + 6];
+    for (int i = 0; i < 3; ++i) C[i + 3 * j] = dot3(A[i], B[j], A[i + 3], B[j + 3], A[i + 6], B[j + 6]);
 }
 __device__ __forceinline__ double det33(const double* m) {
-  return m[0] * (m[4] * m[8] - m[7] * m[5]) - m[3] * (m[1] * m[8] - m[7] * m[2]) + m[6] * (m[1] * m[5] - m[4] * m[2]);
+  return dot3(m[0], cross2(m[4], m[8], m[7], m[5]), -m[3], cross2(m[1], m[8], m[7], m[2]), m[6],
+              cross2(m[1], m[5], m[4], m[2]));
 }
 // math_invert33 (Cramer), math.f90:471-509; returns true on error
 __device__ __forceinline__ bool inv33(const double* A, double* I) {
-  I[0] = A[4] * A[8] - A[7] * A[5];
-  I[1] = -A[1] * A[8] + A[7] * A[2];
-  I[2] = A[1] * A[5] - A[4] * A[2];
-  const double det = A[0] * I[0] + A[3] * I[1] + A[6] * I[2];
+  I[0] = cross2(A[4], A[8], A[7], A[5]);
+  I[1] = cross2(-A[1], A[8], -A[7], A[2]);
+  I[2] = cross2(A[1], A[5], A[4], A[2]);
+  const double det = dot3(A[0], I[0], A[3], I[1], A[6], I[2]);
   if (fabs(det) <= TINY10) return true;
-  I[3] = -A[3] * A[8] + A[6] * A[5];
-  I[4] = A[0] * A[8] - A[6] * A[2];
-  I[5] = -A[0] * A[5] + A[3] * A[2];
-  I[6] = A[3] * A[7] - A[6] * A[4];
-  I[7] = -A[0] * A[7] + A[6] * A[1];
-  I[8] = A[0] * A[4] - A[3] * A[1];
+  I[3] = cross2(-A[3], A[8], -A[6], A[5]);
+  I[4] = cross2(A[0], A[8], A[6], A[2]);
+  I[5] = cross2(-A[0], A[5], -A[3], A[2]);
+  I[6] = cross2(A[3], A[7], A[6], A[4]);
+  I[7] = cross2(-A[0], A[7], -A[6], A[1]);
+  I[8] = cross2(A[0], A[4], A[3], A[1]);
   const double r = 1.0 / det;
 #pragma unroll
   for (int k = 0; k < 9; ++k) I[k] *= r;
@@ -215,16 +221,49 @@ __host__ __device__ inline SysConst make_sys_const(const PhaseConst<NS>& pc, int
   return c;
 }
 
+// Per slip system constants of the Newton loop of a phase without non-Schmid terms (both senses
+// share P_s).  The traceless P_s in eight coordinates: its symmetric part u = (P11, P22, and the
+// symmetric (23), (13), (12) components), its skew part v = ((P23 - P32), (P13 - P31), (P12 - P21)) / 2,
+// so that P33 = -u0 - u1, P23 = u2 + v0, P32 = u2 - v0, and so on.
+struct SchmidConst {
+  double2 u01, u23, u4v0, v12;
+  double2 kin;       // (dot_gamma_0, n)
+  int n_int;         // stress exponent if integral (1..64), else -1
+  int pad[3];
+};
+
+template <int NS>
+__host__ __device__ inline SchmidConst make_schmid_const(const PhaseConst<NS>& pc, int i) {
+  const double* P = pc.P[i];   // column-major: P(r, c) = P[r + 3 c]
+  SchmidConst c;
+  c.u01 = make_double2(P[0], P[4]);
+  c.u23 = make_double2(0.5 * (P[7] + P[5]), 0.5 * (P[6] + P[2]));
+  c.u4v0 = make_double2(0.5 * (P[3] + P[1]), 0.5 * (P[7] - P[5]));
+  c.v12 = make_double2(0.5 * (P[6] - P[2]), 0.5 * (P[3] - P[1]));
+  c.kin = make_double2(pc.dg0[i], pc.n[i]);
+  c.n_int = pc.n_int[i];
+  c.pad[0] = c.pad[1] = c.pad[2] = 0;
+  return c;
+}
+
+// The per-system constants that a stress kernel stages: SchmidConst or (general phases) SysConst.
+template <bool SCHMID>
+using StressConst = typename std::conditional<SCHMID, SchmidConst, SysConst>::type;
+
 // Copies the NS per-system constants from device memory into shared memory: every thread of
 // the block moves 16-byte words of the contiguous array (no per-thread divergent reads of the
 // parameter space).
-template <int NS>
-__device__ __forceinline__ void stage_sys_const(const PhaseConst<NS>& pc, SysConst* sc) {
-  constexpr int WORDS = NS * int(sizeof(SysConst) / sizeof(double2));
-  const double2* __restrict__ src = reinterpret_cast<const double2*>(pc.sys);
+template <int NS, class SC>
+__device__ __forceinline__ void stage_sys_const(const SC* __restrict__ sys, SC* sc) {
+  constexpr int WORDS = NS * int(sizeof(SC) / sizeof(double2));
+  const double2* __restrict__ src = reinterpret_cast<const double2*>(sys);
   double2* dst = reinterpret_cast<double2*>(sc);
   for (int i = threadIdx.x; i < WORDS; i += blockDim.x) dst[i] = src[i];
 }
+template <int NS>
+__device__ __forceinline__ const SysConst* stress_const(const PhaseConst<NS>& pc, SysConst*) { return pc.sys; }
+template <int NS>
+__device__ __forceinline__ const SchmidConst* stress_const(const PhaseConst<NS>& pc, SchmidConst*) { return pc.schmid; }
 
 // Hooke in Mandel notation with Fi = I: S = C66 : sym6(E), E = (Fe^T Fe - I)/2
 // (phase_hooke_SandItsTangents, phase_mechanical_elastic.f90:172-205)
@@ -234,12 +273,12 @@ __device__ __forceinline__ void hooke_S(const PhaseConst<NS>& pc, const double* 
   const double IW = 1.0 / W;                  // 1/WGT_MANDEL(1)
   double E[6];
   // E = 0.5 (Fe^T Fe - I): (11,22,33,23,13,12)
-  E[0] = 0.5 * (Fe[0] * Fe[0] + Fe[1] * Fe[1] + Fe[2] * Fe[2] - 1.0);
-  E[1] = 0.5 * (Fe[3] * Fe[3] + Fe[4] * Fe[4] + Fe[5] * Fe[5] - 1.0);
-  E[2] = 0.5 * (Fe[6] * Fe[6] + Fe[7] * Fe[7] + Fe[8] * Fe[8] - 1.0);
-  E[3] = 0.5 * (Fe[3] * Fe[6] + Fe[4] * Fe[7] + Fe[5] * Fe[8]) * W;
-  E[4] = 0.5 * (Fe[0] * Fe[6] + Fe[1] * Fe[7] + Fe[2] * Fe[8]) * W;
-  E[5] = 0.5 * (Fe[0] * Fe[3] + Fe[1] * Fe[4] + Fe[2] * Fe[5]) * W;
+  E[0] = 0.5 * (dot3(Fe[0], Fe[0], Fe[1], Fe[1], Fe[2], Fe[2]) - 1.0);
+  E[1] = 0.5 * (dot3(Fe[3], Fe[3], Fe[4], Fe[4], Fe[5], Fe[5]) - 1.0);
+  E[2] = 0.5 * (dot3(Fe[6], Fe[6], Fe[7], Fe[7], Fe[8], Fe[8]) - 1.0);
+  E[3] = 0.5 * dot3(Fe[3], Fe[6], Fe[4], Fe[7], Fe[5], Fe[8]) * W;
+  E[4] = 0.5 * dot3(Fe[0], Fe[6], Fe[1], Fe[7], Fe[2], Fe[8]) * W;
+  E[5] = 0.5 * dot3(Fe[0], Fe[3], Fe[1], Fe[4], Fe[2], Fe[5]) * W;
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
     double s = 0.0;
@@ -250,7 +289,7 @@ __device__ __forceinline__ void hooke_S(const PhaseConst<NS>& pc, const double* 
 }
 
 __device__ __forceinline__ double dot6(const double* a, const double* b) {
-  return a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3] + a[4] * b[4] + a[5] * b[5];
+  return fma(a[5], b[5], fma(a[4], b[4], fma(a[3], b[3], dot3(a[0], b[0], a[1], b[1], a[2], b[2]))));
 }
 
 // warp + block reduction of a small vector; result valid in thread 0
