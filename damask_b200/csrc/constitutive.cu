@@ -81,15 +81,13 @@ __device__ __forceinline__ void count_iterations_batch(const Fields* __restrict_
 // one context (grid constants) and the batch kernels (tables of many contexts in device memory)
 // share them.
 
-// begin: F <- F - r, mechanical_restore, first substep control, state-iteration start; returns
-// whether the voxel goes on to an integrateStress
-template <int NS>
-__device__ __forceinline__ bool begin_voxel(const PhaseConst<NS>& pc, const double* __restrict__ hs, double* xs,
-                                            const Numerics& nm, const Fields& f, const PassWork& w, int64_t v,
-                                            double dt, int apply_update, int use_dot0) {
-  constexpr int NST = 2 * NS;
+// F <- F - r (the Richardson/Anderson update of the previous evaluation), phase F, mechanical_restore
+// and the first substep control step (status ITERATING: subStep = r_cutback / r_cutback = 1, nothing to
+// restore beyond the increment-start values, which stay where they are while stepFrac = 0; Lp is kept
+// as warm start); c.nsub = 1 when a substep starts, PH_DONE otherwise
+__device__ __forceinline__ void begin_update(const Numerics& nm, const Fields& f, const PassWork& w, int64_t v,
+                                             int apply_update, VoxelCtl& c) {
   const int64_t N = f.N;
-  // F <- F - r (the Richardson/Anderson update of the previous evaluation), phase F
   double Fn[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
@@ -101,42 +99,52 @@ __device__ __forceinline__ bool begin_voxel(const PhaseConst<NS>& pc, const doub
     f.F[k * N + v] = x;
     Fn[k] = x;
   }
-  // mechanical_restore and the first substep control step (status ITERATING: subStep =
-  // r_cutback / r_cutback = 1, nothing to restore beyond the increment-start values,
-  // which stay where they are while stepFrac = 0; Lp is kept as warm start)
-  VoxelCtl c;
   c.status = 1;
   c.it = 0;
   c.nsub = 0;
   c.nstate = 0;
   c.newton = 0;
+  c.from_start = false;
   c.stepFrac = 0.0;
   c.step = nm.r_cutback * (1.0 / nm.r_cutback);
-  if (!(c.step > nm.r_cutback_min)) {
-    c.phase = PH_DONE;
-  } else {
-    c.nsub = 1;
+  c.phase = PH_DONE;
+  if (!(c.step > nm.r_cutback_min)) return;
+  c.nsub = 1;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      const double f0 = f.F0[k * N + v];
-      w.Fs[k * N + v] = fma(c.step, Fn[k] - f0, f0);
-    }
+  for (int k = 0; k < 9; ++k) {
+    const double f0 = f.F0[k * N + v];
+    w.Fs[k * N + v] = fma(c.step, Fn[k] - f0, f0);
+  }
+}
+
+// begin: begin_update and the state-iteration start; returns whether the voxel goes on to an
+// integrateStress
+template <int NS>
+__device__ __forceinline__ bool begin_voxel(const PhaseConst<NS>& pc, const double* __restrict__ hs, double* xs,
+                                            const Numerics& nm, const Fields& f, const PassWork& w, int64_t v,
+                                            double dt, int apply_update, int use_dot0) {
+  constexpr int NST = 2 * NS;
+  const int64_t N = f.N;
+  VoxelCtl c;
+  begin_update(nm, f, w, v, apply_update, c);
+  if (c.nsub) {
     // start of the state iteration (integrateStateFPI:614-620) at S0 and state0.  The rate
-    // depends on the increment-start values only, so every evaluation of an increment after
-    // the first reads it back (use_dot0) instead of evaluating the kinetics and hardening.
-    bool bad = false;
+    // depends on the increment-start values only, so it is evaluated in the first evaluation of an
+    // increment and kept in dot0; the passes form the state that it leads to, state0 + dot0 step dt,
+    // where they need it (negative step: see VoxelCtl), so neither it nor a copy of the rate is
+    // written here.  A NaN among the rates is marked in the first of them.
+    bool bad;
     if (use_dot0) {
-#pragma unroll 12
-      for (int i = 0; i < NST; ++i) {
-        const double d = w.dot0[i * N + v];
-        bad |= isnan(d);
-        xs[i * pass_threads<NS>()] = d;
-      }
+      bad = isnan(w.dot0[v]);
     } else {
       double s0[6];
 #pragma unroll
       for (int k = 0; k < 6; ++k) s0[k] = f.S0[k * N + v];
-      bad = dot_state_slots<NS>(pc, hs, s0, f.state0, N, v, xs, nullptr, 0);
+      bad = dot_state_slots<NS>(pc, hs, s0, [&](int i) { return f.state0[i * N + v]; }, xs, nullptr, 0);
+      if (bad) {
+        xs[0] = nan("");
+        if (w.dot0_nan) *w.dot0_nan = 1;
+      }
 #pragma unroll 12
       for (int i = 0; i < NST; ++i) w.dot0[i * N + v] = xs[i * pass_threads<NS>()];
     }
@@ -156,15 +164,8 @@ __device__ __forceinline__ bool begin_voxel(const PhaseConst<NS>& pc, const doub
       c.phase = PH_CTRL;
       advance<NS>(pc, hs, nm, f, w, v, dt, c, xs, nullptr, 0);
     } else {
-      const double dts = c.step * dt;
-      double* D0 = w.D + v;                               // dotState generation 0
-#pragma unroll 12
-      for (int i = 0; i < NST; ++i) {
-        const double d = xs[i * pass_threads<NS>()];
-        f.state[i * N + v] = fma(d, dts, f.state0[i * N + v]);
-        D0[i * N] = d;
-      }
       // S is written by the first successful integrateStress (a failure restores S0)
+      c.from_start = true;
       c.phase = PH_STRESS;
     }
   }
@@ -183,7 +184,8 @@ __device__ __forceinline__ int stress_voxel(const PhaseConst<NS>& pc, const SC* 
   int dnewton = 0;
   // every load of the voxel at once (one exposure of the memory latency), the substep's Fp0
   // speculatively that of the first substep (see sub_start)
-  const double frac = w.sub[v], step = w.sub[N + v];
+  const double frac = w.sub[v], step_c = w.sub[N + v], step = fabs(step_c);
+  const bool fresh = step_c < 0.0 && w.ctl[2 * N + v] == 0;   // the state is state0 + dot0 step dt
   double Lp[9], F[9], Fp0[9], xi[NS];
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
@@ -191,8 +193,13 @@ __device__ __forceinline__ int stress_voxel(const PhaseConst<NS>& pc, const SC* 
     F[k] = w.Fs[k * N + v];
     Fp0[k] = f.Fp0[k * N + v];
   }
+  if (fresh) {
 #pragma unroll
-  for (int s = 0; s < NS; ++s) xi[s] = f.state[s * N + v];
+    for (int s = 0; s < NS; ++s) xi[s] = fma(w.dot0[s * N + v], step * dt, f.state0[s * N + v]);
+  } else {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) xi[s] = f.state[s * N + v];
+  }
   const double* Fp0g = f.Fp0 + v;
   if (frac != 0.0) {
     Fp0g = w.Fp0s + v;
@@ -257,6 +264,29 @@ constitutive_begin_kernel(const __grid_constant__ PhaseConst<NS> pc, const __gri
   __syncthreads();
   const int64_t v = v_begin + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool keep = v < v_end && begin_voxel<NS>(pc, hs, xs, nm, f, w, v, dt, apply_update, use_dot0);
+  append(w.list_out, w.count_out, keep, v);
+}
+
+// The same once the increment-start rates are stored and none of them is NaN (use_dot0 of
+// begin_voxel): no kinetics, no hardening and no slots, so the kernel streams its planes at full
+// occupancy.
+template <int NS>
+__global__ void __launch_bounds__(256)
+constitutive_restart_kernel(const __grid_constant__ Numerics nm, const __grid_constant__ Fields f,
+                            const __grid_constant__ PassWork w, int apply_update, int64_t v_begin, int64_t v_end) {
+  const int64_t v = v_begin + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  bool keep = false;
+  if (v < v_end) {
+    VoxelCtl c;
+    begin_update(nm, f, w, v, apply_update, c);
+    if (c.nsub) {
+      c.from_start = true;
+      c.phase = PH_STRESS;
+    }
+    store_ctl(w, f.N, v, c);
+    keep = c.phase == PH_STRESS;
+    if (!keep) finish_voxel(f, v, c);
+  }
   append(w.list_out, w.count_out, keep, v);
 }
 
@@ -413,16 +443,21 @@ __global__ void batch_flip_kernel(int* count_done, const int* count_next, int* i
 
 template <int NS>
 cudaError_t launch_constitutive_begin(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f,
-                                      const PassWork& w, double dt, int apply_update, int use_dot0, int64_t v_begin,
+                                      const PassWork& w, double dt, int apply_update, BeginMode mode, int64_t v_begin,
                                       int64_t v_end, cudaStream_t s) {
+  if (v_end <= v_begin) return cudaSuccess;
+  if (mode == BEGIN_RESTART) {
+    constitutive_restart_kernel<NS><<<int((v_end - v_begin + 255) / 256), 256, 0, s>>>(nm, f, w, apply_update, v_begin,
+                                                                                     v_end);
+    return cudaGetLastError();
+  }
   const size_t smem = (hard_smem_doubles<NS>() + size_t(2 * NS) * pass_threads<NS>()) * sizeof(double);
   cudaError_t e = cudaFuncSetAttribute(constitutive_begin_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        int(smem));
   if (e != cudaSuccess) return e;
-  if (v_end <= v_begin) return cudaSuccess;
   const int nb = int((v_end - v_begin + pass_threads<NS>() - 1) / pass_threads<NS>());
-  constitutive_begin_kernel<NS><<<nb, pass_threads<NS>(), smem, s>>>(pc, nm, f, w, dt, apply_update, use_dot0, v_begin,
-                                                                v_end);
+  constitutive_begin_kernel<NS><<<nb, pass_threads<NS>(), smem, s>>>(pc, nm, f, w, dt, apply_update,
+                                                                mode == BEGIN_STORED ? 1 : 0, v_begin, v_end);
   return cudaGetLastError();
 }
 
@@ -573,7 +608,7 @@ cudaError_t build_batch_pass_graph(const PhaseConst<NS>& pc, const Numerics& nm,
 
 #define DMK_INSTANTIATE(NS)                                                                                         \
   template cudaError_t launch_constitutive_begin<NS>(const PhaseConst<NS>&, const Numerics&, const Fields&,          \
-                                                     const PassWork&, double, int, int, int64_t, int64_t,          \
+                                                     const PassWork&, double, int, BeginMode, int64_t, int64_t,    \
                                                      cudaStream_t);                                                 \
   template cudaError_t launch_constitutive_pass<NS>(const PhaseConst<NS>&, const Numerics&, const Fields&,           \
                                                     const PassWork&, double, const int*, int64_t, cudaStream_t,    \

@@ -43,6 +43,8 @@ __device__ __forceinline__ void load_ctl(const PassWork& w, int64_t N, int64_t v
   c.newton = w.ctl[5 * N + v];
   c.stepFrac = w.sub[v];
   c.step = w.sub[N + v];
+  c.from_start = c.step < 0.0;
+  c.step = fabs(c.step);
 }
 __device__ __forceinline__ void store_ctl(const PassWork& w, int64_t N, int64_t v, const VoxelCtl& c) {
   w.ctl[v] = c.phase;
@@ -52,7 +54,7 @@ __device__ __forceinline__ void store_ctl(const PassWork& w, int64_t N, int64_t 
   w.ctl[4 * N + v] = c.nstate;
   w.ctl[5 * N + v] = c.newton;
   w.sub[v] = c.stepFrac;
-  w.sub[N + v] = c.step;
+  w.sub[N + v] = c.from_start ? -c.step : c.step;
 }
 
 // Solves A x = b for a row-major n x n A (overwritten with R) by Householder QR:
@@ -583,16 +585,16 @@ __device__ __forceinline__ void stage_hardening(const PhaseConst<NS>& pc, double
   for (int i = threadIdx.x; i < NS * NS; i += blockDim.x) hs[i] = pc.hmat[i];
 }
 
-// phenopowerlaw_dotState (Fi = I => Mp = S; no twins => sumF = 0) at the stored
-// stress and state of voxel v, written to this thread's slots: xi rates first, then
+// phenopowerlaw_dotState (Fi = I => Mp = S; no twins => sumF = 0) at the given
+// stress and state (state(i): value i of the voxel), written to this thread's slots: xi rates first, then
 // |dot_gamma|.  hs: the hardening matrix (shared memory, or device memory read with uniform
 // addresses).  adg_in (element s at adg_in[s * adg_stride]), when given, holds |dot_gamma| at
 // this stress and state already (the kinetics of the converged integrateStress); otherwise
 // the kinetics are evaluated.  Returns true if any rate is NaN.
-template <int NS>
-__device__ bool dot_state_slots(const PhaseConst<NS>& pc, const double* __restrict__ hs, const double s6[6],
-                                const double* __restrict__ state, int64_t N, int64_t v, double* xs,
-                                const double* adg_in, int64_t adg_stride) {
+template <int NS, class State>
+__device__ __forceinline__ bool dot_state_slots(const PhaseConst<NS>& pc, const double* __restrict__ hs,
+                                                const double s6[6], const State& state, double* xs,
+                                                const double* adg_in, int64_t adg_stride) {
   double adg[NS];
   if (adg_in) {
 #pragma unroll
@@ -602,13 +604,13 @@ __device__ bool dot_state_slots(const PhaseConst<NS>& pc, const double* __restri
     for (int s = 0; s < NS; ++s) {
       const double tp = dot6(s6, pc.p6[0][s]), tn = dot6(s6, pc.p6[1][s]);
       const double tmax = tp > tn ? tp : tn;
-      adg[s] = fabs(pc.dg0[s] * powr(tmax / state[s * N + v], pc.n[s], pc.n_int[s]));
+      adg[s] = fabs(pc.dg0[s] * powr(tmax / state(s), pc.n[s], pc.n_int[s]));
     }
   }
   bool bad = false;
   // xi of every system into the slots first, so that the loads overlap
 #pragma unroll 8
-  for (int l = 0; l < NS; ++l) xs[l * pass_threads<NS>()] = state[l * N + v];
+  for (int l = 0; l < NS; ++l) xs[l * pass_threads<NS>()] = state(l);
 #pragma unroll 2
   for (int l = 0; l < NS; ++l) {
     const double x = fma(-xs[l * pass_threads<NS>()], pc.ixiinf[l], 1.0);  // 1 - xi/xi_inf
@@ -675,6 +677,7 @@ __device__ void advance(const PhaseConst<NS>& pc, const double* __restrict__ hs,
     if (guard > 4096) { c.status = 3; c.phase = PH_DONE; break; }
     if (c.phase == PH_CTRL) {
       // substep control, phase_mechanical.f90:1040-1080
+      c.from_start = false;
       bool todo;
       if (c.status == 0) {
         c.stepFrac = c.stepFrac + c.step;
@@ -719,17 +722,24 @@ __device__ void advance(const PhaseConst<NS>& pc, const double* __restrict__ hs,
       if (!after_stress)
 #pragma unroll
         for (int k = 0; k < 6; ++k) s6[k] = f.S[k * N + v];
-      const bool bad = dot_state_slots<NS>(pc, hs, s6, f.state, N, v, xs, after_stress ? adg : nullptr, adg_stride);
       const double dts = c.step * dt;
+      // the first update after a start from the increment-start values
+      const bool fresh = after_stress && c.from_start && c.it == 1;
+      const double* st0 = sub_start(f, w, c.stepFrac).st0 + v;
+      const double* stv = fresh ? w.dot0 + v : f.state + v;
+      auto state = [&](int i) {
+        const double x = stv[i * N];
+        return fresh ? fma(x, dts, st0[i * N]) : x;
+      };
+      const bool bad = dot_state_slots<NS>(pc, hs, s6, state, xs, after_stress ? adg : nullptr, adg_stride);
       if (c.phase == PH_DOT0) {
         // integrateStateFPI:616-620
         if (bad) { c.status = 3; c.phase = PH_CTRL; continue; }   // STATUS_FAIL_PHASE_MECHANICAL_STATE
         double* D0 = dot_gen(w, 0, NST, N) + v;
-        const double* st0 = sub_start(f, w, c.stepFrac).st0;
 #pragma unroll 12
         for (int i = 0; i < NST; ++i) {
           const double d = xs[i * pass_threads<NS>()];
-          f.state[i * N + v] = fma(d, dts, st0[i * N + v]);
+          f.state[i * N + v] = fma(d, dts, st0[i * N]);
           D0[i * N] = d;
         }
         c.it = 0;
@@ -739,34 +749,42 @@ __device__ void advance(const PhaseConst<NS>& pc, const double* __restrict__ hs,
         if (bad) { c.phase = PH_CTRL; continue; }
         // generations: dotState of the last iteration (it - 1) and the one before (it - 2,
         // whose storage receives the damped rate of this iteration)
-        const double* L1 = dot_gen(w, c.it + 1, NST, N) + v;
+        const double* L1 = fresh ? w.dot0 + v : dot_gen(w, c.it + 1, NST, N) + v;
         double* L2 = dot_gen(w, c.it, NST, N) + v;
+        const double* L2r = c.from_start && c.it == 2 ? w.dot0 + v : L2;
         double d01 = 0.0, d12 = 0.0, d22 = 0.0;
 #pragma unroll 24
         for (int i = 0; i < NST; ++i) {
           const double d = xs[i * pass_threads<NS>()];
           const double l1 = L1[i * N];                                 // dotState_last(:,1)
-          const double l2 = c.it > 1 ? L2[i * N] : 0.0;               // dotState_last(:,2)
+          const double l2 = c.it > 1 ? L2r[i * N] : 0.0;              // dotState_last(:,2)
           const double a = d - l1, b = l1 - l2;
           d12 = fma(a, b, d12);
           d22 = fma(b, b, d22);
           d01 = fma(d, l1, d01);
         }
         const double zeta = damper(d01, d12, d22);
-        const double* st0 = sub_start(f, w, c.stepFrac).st0;
+        if (zeta != 1.0)                                              // rarely: the damped rate
+#pragma unroll 12
+          for (int i = 0; i < NST; ++i)
+            xs[i * pass_threads<NS>()] = fma(xs[i * pass_threads<NS>()], zeta, L1[i * N] * (1.0 - zeta));
         bool conv = true;
 #pragma unroll 12
         for (int i = 0; i < NST; ++i) {
-          const double l1 = L1[i * N];
-          const double d = fma(xs[i * pass_threads<NS>()], zeta, l1 * (1.0 - zeta));
-          const double st = f.state[i * N + v];
-          const double r = fma(-d, dts, st - st0[i * N + v]);
+          const double d = xs[i * pass_threads<NS>()];
+          const double x0 = st0[i * N];
+          const double x = stv[i * N];
+          const double st = fresh ? fma(x, dts, x0) : x;
+          const double r = fma(-d, dts, st - x0);
           const double stn = st - r;
           f.state[i * N + v] = stn;
-          L2[i * N] = d;
           const double atol = i < NS ? pc.atol_xi : pc.atol_gamma;
           conv = conv && (fabs(r) <= fmax(atol, nm.eps_rel_state * fabs(stn)));
         }
+        // the rate of this iteration is read by the next ones only
+        if (!conv && c.it < nm.N_iter_state_max)
+#pragma unroll 12
+          for (int i = 0; i < NST; ++i) L2[i * N] = xs[i * pass_threads<NS>()];
         c.phase = (conv || c.it >= nm.N_iter_state_max) ? PH_CTRL : PH_STRESS;
       }
     }

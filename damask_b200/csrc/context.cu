@@ -138,6 +138,7 @@ struct dmk_ctx {
   int* pctl = nullptr;           // 6 planes of per-voxel control integers
   double* dot0 = nullptr;        // 2 NS planes: dotState at (S0, state0), see dot0_valid
   bool dot0_valid = false;       // dot0 holds the rates of the current increment-start values
+  bool dot0_finite = false;      // and none of them is known to be NaN (read back after their evaluation)
   // The voxels are split into PASS_CHUNKS chunks whose pass loops run on their own streams,
   // so that the latency-bound control kernel of one chunk overlaps the compute-bound stress
   // kernel of another.  Per chunk: two voxel lists alternating between passes, their counts.
@@ -203,6 +204,7 @@ PassWork pass_work(dmk_ctx* c, int half, int out) {
   w.dot0 = c->dot0;
   w.sub = w.adg + int64_t(c->NS) * N;
   w.ctl = c->pctl;
+  w.dot0_nan = c->pcount + 2 * PASS_CHUNKS;
   w.list_out = c->plist[half][out];
   w.count_out = c->pcount + 2 * half + out;
   return w;
@@ -217,6 +219,8 @@ int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, d
     lo[h] = c->N * h / K;
     hi[h] = c->N * (h + 1) / K;
   }
+  const BeginMode mode = !c->dot0_valid ? BEGIN_EVALUATE : c->dot0_finite ? BEGIN_RESTART : BEGIN_STORED;
+  if (mode == BEGIN_EVALUATE) CK(cudaMemsetAsync(c->pcount + 2 * PASS_CHUNKS, 0, sizeof(int), c->stream));
   // the other streams start after everything queued on the first
   CK(cudaEventRecord(c->fork, c->stream));
   for (int h = 1; h < K; ++h) CK(cudaStreamWaitEvent(c->cstream[h], c->fork, 0));
@@ -226,8 +230,7 @@ int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, d
     // pass 0: restore and control up to the first integrateStress of every voxel of the chunk
     cur[h] = 0;
     CK(cudaMemsetAsync(c->pcount + 2 * h, 0, 2 * sizeof(int), c->cstream[h]));
-    CKL(launch_constitutive_begin<NS>(pc, c->nm, f, pass_work(c, h, 0), dt, apply, c->dot0_valid ? 1 : 0, lo[h], hi[h],
-                                      c->cstream[h]));
+    CKL(launch_constitutive_begin<NS>(pc, c->nm, f, pass_work(c, h, 0), dt, apply, mode, lo[h], hi[h], c->cstream[h]));
     CK(cudaMemcpyAsync(c->hcount + h, c->pcount + 2 * h, sizeof(int), cudaMemcpyDeviceToHost, c->cstream[h]));
     ++c->passes;
     active[h] = hi[h] > lo[h];
@@ -259,6 +262,12 @@ int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, d
   for (int h = 1; h < K; ++h) {
     CK(cudaEventRecord(c->join[h], c->cstream[h]));
     CK(cudaStreamWaitEvent(c->stream, c->join[h], 0));
+  }
+  if (mode == BEGIN_EVALUATE) {
+    CK(cudaMemcpyAsync(c->hcount + PASS_CHUNKS, c->pcount + 2 * PASS_CHUNKS, sizeof(int), cudaMemcpyDeviceToHost,
+                       c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    c->dot0_finite = c->hcount[PASS_CHUNKS] == 0;
   }
   return 0;
 }
@@ -1126,7 +1135,7 @@ int dmk_mech_init(dmk_ctx** out, const int cells[3], const double geomSize[3], c
       (rc = dalloc(&c->sc, 1)) || (rc = dalloc(&c->tan_out, 245)) || (rc = dalloc(&c->tan_idx, 2)) ||
       (rc = dalloc(&c->pw, pass_work_doubles(N, c->NS))) || (rc = dalloc(&c->pctl, 6 * size_t(N))) ||
       (rc = dalloc(&c->dot0, size_t(NST) * N)) ||
-      (rc = dalloc(&c->pcount, 2 * PASS_CHUNKS)) || (rc = dalloc(&c->xp, 3 * size_t(N))) ||
+      (rc = dalloc(&c->pcount, 2 * PASS_CHUNKS + 1)) || (rc = dalloc(&c->xp, 3 * size_t(N))) ||
       (rc = dalloc(&c->xn, 3 * size_t(node_count(c)))) || (rc = dalloc(&c->favg, 9)))
     return bail(rc);
   // a chunk of at least 65536 voxels keeps a pass kernel wide enough to be worth its own stream
@@ -1137,7 +1146,7 @@ int dmk_mech_init(dmk_ctx** out, const int cells[3], const double geomSize[3], c
     const size_t len = size_t((N + h) / (h + 1));
     if ((rc = dalloc(&c->plist[h][0], len)) || (rc = dalloc(&c->plist[h][1], len))) return bail(rc);
   }
-  if (cudaMallocHost(reinterpret_cast<void**>(&c->hcount), PASS_CHUNKS * sizeof(int)) != cudaSuccess) {
+  if (cudaMallocHost(reinterpret_cast<void**>(&c->hcount), (PASS_CHUNKS + 1) * sizeof(int)) != cudaSuccess) {
     c->hcount = nullptr;
     return bail(fail(DMK_ERR_CUDA, "cudaMallocHost failed"));
   }
@@ -1392,7 +1401,7 @@ int dmk_materialpoint_forward(dmk_ctx* c) {
   CK(cudaMemcpyAsync(c->Lp0, c->Lp, b9, cudaMemcpyDeviceToDevice, c->stream));
   CK(cudaMemcpyAsync(c->S0, c->S, b6, cudaMemcpyDeviceToDevice, c->stream));
   CK(cudaMemcpyAsync(c->state0, c->state, bs, cudaMemcpyDeviceToDevice, c->stream));
-  c->dot0_valid = false;                                   // new increment-start values
+  c->dot0_valid = c->dot0_finite = false;                  // new increment-start values
   return 0;
 }
 
@@ -1874,6 +1883,7 @@ void pack_host(dmk_ctx* c, std::vector<double>& h) {
   if (!SAVE) {
     for (int k = 0; k < 9; ++k) c->stress_mask[k] = int(ints[k]);
     c->dot0_valid = ints[9] != 0.0;
+    c->dot0_finite = false;
   }
 }
 
@@ -2670,6 +2680,7 @@ int batch_solution_impl(dmk_batch* b, const int* which, int nw, dmk_solution_sta
       const BatchScal& hs = b->h_scal[r];
       if (hs.status == 0) std::swap(c->P, c->Pnew);
       c->dot0_valid = true;
+      c->dot0_finite = false;
       ++S.evals;
       if (S.nsl > 0) {
         const double* dots = b->h_dots + size_t(r) * BATCH_DOTS;

@@ -88,16 +88,21 @@ struct PassWork {
   double* D;       // 2 x 2 NS: (damped) dotState of the last two state iterations
   double* adg;     // NS: |dot_gamma| at the stress of the last converged integrateStress
   double* dot0;    // 2 NS: dotState at the increment-start stress and state (S0, state0)
-  double* sub;     // 2: stepFrac (subFrac), step (subStep)
+  double* sub;     // 2: stepFrac (subFrac), step (subStep; negative: VoxelCtl::from_start)
   int* ctl;        // 6: phase, status, state iteration, substeps, state iterations total, Newton total
+  int* dot0_nan;   // set when an increment-start rate is NaN (null in batches)
   int* list_out;   // voxels that continue into the next pass
   int* count_out;  // number of entries appended to list_out
 };
 
 enum : int { PH_CTRL = 0, PH_DOT0 = 1, PH_STRESS = 2, PH_DOT1 = 3, PH_DONE = 4 };
 
+// from_start: the running state iteration started from the increment-start state and rate (the first
+// attempt of the first substep); it is kept as the sign of the stored step.  Its start state, state0 +
+// dot0 step dt, and its generation-0 rate, dot0, are then not stored but formed from these planes.
 struct VoxelCtl {
   int phase, status, it, nsub, nstate, newton;
+  bool from_start;
   double stepFrac, step;
 };
 

@@ -77,9 +77,11 @@ struct Numerics2 {
 };
 
 // constitutive passes (constitutive.cu)
+// the increment-start rates: evaluated and stored, read back, or read back with none of them NaN
+enum BeginMode : int { BEGIN_EVALUATE = 0, BEGIN_STORED = 1, BEGIN_RESTART = 2 };
 template <int NS>
 cudaError_t launch_constitutive_begin(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f,
-                                      const PassWork& w, double dt, int apply_update, int use_dot0, int64_t v_begin,
+                                      const PassWork& w, double dt, int apply_update, BeginMode mode, int64_t v_begin,
                                       int64_t v_end, cudaStream_t s);
 // variant: the stress kernel's register bound (stress_variant_blocks: resident blocks per SM)
 template <int NS>
