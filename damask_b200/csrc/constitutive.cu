@@ -334,6 +334,44 @@ constitutive_control_kernel(const __grid_constant__ PhaseConst<NS> pc, const __g
   append(w.list_out, w.count_out, keep, v);
 }
 
+// One evaluation of a small grid in one launch: every voxel's begin, and its stress integrations and
+// control steps one after the other until it is done.  No voxel lists and no host between passes.  With
+// every voxel resident at once there is nothing that the lists' compaction could gain, and what
+// bounds such a grid is the chain of one voxel, launches and host round trips.
+template <int NS, bool SCHMID>
+struct FusedShape : StressShape<NS, SCHMID, 2> {
+  using Base = StressShape<NS, SCHMID, 2>;
+  static constexpr size_t smem = Base::smem + sizeof(double) * hard_smem_doubles<NS>();
+  static_assert(Base::threads == pass_threads<NS>(), "the control step's slots share the stress slots' stride");
+};
+template <int NS, bool SCHMID>
+__global__ void __launch_bounds__(FusedShape<NS, SCHMID>::threads, 2)
+constitutive_fused_kernel(const __grid_constant__ PhaseConst<NS> pc, const __grid_constant__ Numerics nm,
+                          const __grid_constant__ Fields f, const __grid_constant__ PassWork w, double dt,
+                          int apply_update, int use_dot0) {
+  using Shape = FusedShape<NS, SCHMID>;
+  extern __shared__ double2 smem2[];
+  auto* sc = reinterpret_cast<StressConst<SCHMID>*>(smem2);
+  double* const staged = reinterpret_cast<double*>(sc + NS);
+  double* xs = staged + hard_smem_doubles<NS>() + threadIdx.x;
+  const double* hs = pc.hmat;
+  stage_sys_const<NS>(stress_const(pc, sc), sc);
+  if constexpr (hard_smem_doubles<NS>() > 0) {
+    stage_hardening<NS>(pc, staged);
+    hs = staged;
+  }
+  __syncthreads();
+  const int64_t v = int64_t(blockIdx.x) * Shape::threads + threadIdx.x;
+  int nstate = 0, newton = 0;
+  bool keep = v < f.N && begin_voxel<NS>(pc, hs, xs, nm, f, w, v, dt, apply_update, use_dot0);
+  while (keep) {
+    newton += stress_voxel<NS, Shape>(pc, sc, xs, nm, f, w, v, dt);
+    ++nstate;
+    keep = control_voxel<NS>(pc, hs, xs, nm, f, w, v, dt);
+  }
+  count_iterations(f.counters, nstate, newton);
+}
+
 // ------------------------------------------------------------------ batch kernels
 // The passes of many contexts of one phase.  Items are the voxels of all contexts, numbered context
 // after context (context r owns items [off[r], off[r + 1])); the lists hold item numbers.  Every
@@ -490,6 +528,30 @@ cudaError_t launch_stress(const PhaseConst<NS>& pc, const Numerics& nm, const Fi
 }
 }  // namespace
 
+namespace {
+template <int NS, bool SCHMID>
+cudaError_t launch_fused_as(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f, const PassWork& w, double dt,
+                            int apply_update, int use_dot0, cudaStream_t s) {
+  using Shape = FusedShape<NS, SCHMID>;
+  cudaError_t e = cudaFuncSetAttribute(constitutive_fused_kernel<NS, SCHMID>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(Shape::smem));
+  if (e != cudaSuccess) return e;
+  const int nb = int((f.N + Shape::threads - 1) / Shape::threads);
+  constitutive_fused_kernel<NS, SCHMID><<<nb, Shape::threads, Shape::smem, s>>>(pc, nm, f, w, dt, apply_update, use_dot0);
+  return cudaGetLastError();
+}
+}  // namespace
+
+// voxels up to which an evaluation runs as one launch: two resident blocks on every SM
+int64_t fused_voxels(int ns, int nsm) { return int64_t(nsm) * 2 * (ns > 24 ? 64 : PASS_THREADS); }
+
+template <int NS>
+cudaError_t launch_constitutive_fused(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f, const PassWork& w,
+                                      double dt, int apply_update, int use_dot0, cudaStream_t s) {
+  return pc.schmid ? launch_fused_as<NS, true>(pc, nm, f, w, dt, apply_update, use_dot0, s)
+                   : launch_fused_as<NS, false>(pc, nm, f, w, dt, apply_update, use_dot0, s);
+}
+
 template <int NS>
 cudaError_t launch_constitutive_pass(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f,
                                      const PassWork& w, double dt, const int* list_in, int64_t n_in, cudaStream_t s,
@@ -607,6 +669,8 @@ cudaError_t build_batch_pass_graph(const PhaseConst<NS>& pc, const Numerics& nm,
 }
 
 #define DMK_INSTANTIATE(NS)                                                                                         \
+  template cudaError_t launch_constitutive_fused<NS>(const PhaseConst<NS>&, const Numerics&, const Fields&,          \
+                                                     const PassWork&, double, int, int, cudaStream_t);              \
   template cudaError_t launch_constitutive_begin<NS>(const PhaseConst<NS>&, const Numerics&, const Fields&,          \
                                                      const PassWork&, double, int, BeginMode, int64_t, int64_t,    \
                                                      cudaStream_t);                                                 \

@@ -149,6 +149,12 @@ struct dmk_ctx {
   int stress_variant = 0;        // register bound of the stress kernel (stress_variant_blocks); dmk_autotune
   int* pcount = nullptr;         // [2 h + k]: entries appended to plist[h][k]
   int* hcount = nullptr;         // pinned host copies of the current counts of the chunks
+  // what the host reads after each residual evaluation, in pinned memory
+  struct Readback {
+    SolverScalars sc;
+    double dots[4 * AA_MAX];
+  };
+  Readback* hread = nullptr;
   int64_t passes = 0;            // constitutive passes launched (all evaluations)
 
   // device checkpoints (dmk_checkpoint_save / _restore): per slot, the per-voxel state and the
@@ -213,6 +219,12 @@ size_t pass_work_doubles(int64_t N, int NS) { return size_t(N) * size_t(36 + 7 *
 
 template <int NS>
 int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, double dt, int apply) {
+  if (c->N <= fused_voxels(NS, c->nsm)) {
+    CKL(launch_constitutive_fused<NS>(pc, c->nm, f, pass_work(c, 0, 0), dt, apply, c->dot0_valid ? 1 : 0, c->stream));
+    ++c->passes;
+    c->dot0_valid = true;
+    return 0;
+  }
   const int K = c->nchunks;
   int64_t lo[PASS_CHUNKS], hi[PASS_CHUNKS];
   for (int h = 0; h < K; ++h) {
@@ -537,26 +549,35 @@ int make_plans(dmk_ctx* c) {
 }
 
 // One constitutive sweep + commit of P (homogenization_mechanical_response + the P part of
-// utilities_constitutiveResponse).  On a failed sweep the previous P field is kept (the
-// reference skips mechanical_homogenize when any cell fails, homogenization.f90:343).
-int evaluate_constitutive(dmk_ctx* c, double dt, const double* r, int apply, int* status_out,
-                          const double* Fsrc = nullptr) {
+// utilities_constitutiveResponse), queued on the stream.  On a failed sweep the previous P field is
+// kept (the reference skips mechanical_homogenize when any cell fails, homogenization.f90:343), which
+// is decided on the device: the status stays in c->status, the sweep's time between ev[0] and ev[1].
+int enqueue_constitutive(dmk_ctx* c, double dt, const double* r, int apply, const double* Fsrc = nullptr) {
   CK(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
   Fields f = make_fields(c, r);
   if (Fsrc) f.Fsol = const_cast<double*>(Fsrc);   // read only when apply == 0
   CK(cudaEventRecord(c->ev[0], c->stream));
   if (int rc = run_constitutive(c, f, dt, apply)) return rc;
   CK(cudaEventRecord(c->ev[1], c->stream));
-  int st = 0;
-  CK(cudaMemcpyAsync(&st, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  std::swap(c->P, c->Pnew);
+  CKL(launch_sum9(c->P, c->N, c->partials, c->stream, c->status, c->Pnew));   // <P> of the committed stress field
+  return 0;
+}
+// the time of the last sweep, once the stream has passed it
+int add_constitutive_ms(dmk_ctx* c) {
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
   c->last_ms[0] += ms;
-  if (st == 0) std::swap(c->P, c->Pnew);
-  CKL(launch_sum9(c->P, c->N, c->partials, c->stream));   // <P> of the committed (or kept) stress field
-  *status_out = st;
   return 0;
+}
+// the same, waiting for it and its status
+int evaluate_constitutive(dmk_ctx* c, double dt, const double* r, int apply, int* status_out,
+                          const double* Fsrc = nullptr) {
+  if (int rc = enqueue_constitutive(c, dt, r, apply, Fsrc)) return rc;
+  CK(cudaMemcpyAsync(c->hcount, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  *status_out = c->hcount[0];
+  return add_constitutive_ms(c);
 }
 
 // dP/dF of every voxel from the stored state: C_volAvg and C_minMaxAvg (grid_utilities.f90:171-202)
@@ -1150,6 +1171,10 @@ int dmk_mech_init(dmk_ctx** out, const int cells[3], const double geomSize[3], c
     c->hcount = nullptr;
     return bail(fail(DMK_ERR_CUDA, "cudaMallocHost failed"));
   }
+  if (cudaMallocHost(reinterpret_cast<void**>(&c->hread), sizeof(dmk_ctx::Readback)) != cudaSuccess) {
+    c->hread = nullptr;
+    return bail(fail(DMK_ERR_CUDA, "cudaMallocHost failed"));
+  }
   if (cudaMallocHost(reinterpret_cast<void**>(&c->tan_host), 247 * sizeof(double)) != cudaSuccess) {
     c->tan_host = nullptr;
     return bail(fail(DMK_ERR_CUDA, "cudaMallocHost failed"));
@@ -1313,19 +1338,18 @@ int dmk_mech_solution(dmk_ctx* c, dmk_solution_state* out) {
   const int nspec = gamma_div_blocks(c->cells[0], c->cells[1], c->cells[2]);
   bool fp32 = mixed;
   int evals = 0, reason = 0;
-  SolverScalars hs;
+  SolverScalars& hs = c->hread->sc;
   int count = 0;                        // Anderson history pairs created so far
   std::vector<double> G(size_t(m > 0 ? m : 1) * (m > 0 ? m : 1), 0.0), bvec;
   std::vector<int> slots_b;             // slots that bvec refers to (oldest -> newest)
-  double dots[4 * AA_MAX];
+  double* const dots = c->hread->dots;
   int new_slot = -1;
 
   // One residual evaluation at the current Fsol (apply: fuse F <- F - r into the sweep).
   // Leaves r (FP64) and the convergence decision in hs; with Anderson also the inner
   // products of the new residual with the history.
   auto evaluate = [&](int apply) -> int {
-    int st = 0;
-    if (int e = evaluate_constitutive(c, c->dt, apply ? c->r : nullptr, apply, &st)) return e;
+    if (int e = enqueue_constitutive(c, c->dt, apply ? c->r : nullptr, apply)) return e;
     ++evals;
     CKL(launch_aim(c->sc, c->partials, nblocks_const(c), c->wgt, 1, c->stream));
     for (int pass = 0; pass < 2; ++pass) {
@@ -1352,6 +1376,8 @@ int dmk_mech_solution(dmk_ctx* c, dmk_solution_state* out) {
       float ms = 0.f;
       CK(cudaEventElapsedTime(&ms, c->ev[2], c->ev[3]));
       c->last_ms[1] += ms;
+      if (pass == 0)
+        if (int e = add_constitutive_ms(c)) return e;
       if (nsl > 0) {
         bvec.assign(nsl, 0.0);
         for (int q = 0; q < nsl; ++q) {
@@ -1828,6 +1854,7 @@ void dmk_destroy(dmk_ctx* c) {
     for (int* p : l)
       if (p) cudaFree(p);
   if (c->hcount) cudaFreeHost(c->hcount);
+  if (c->hread) cudaFreeHost(c->hread);
   if (c->tan_host) cudaFreeHost(c->tan_host);
   for (auto e : c->ev)
     if (e) cudaEventDestroy(e);

@@ -15,7 +15,7 @@
 namespace dmk {
 
 // partial sums of a 9-plane field (used when the stale P field is kept after a failure)
-__device__ __forceinline__ void sum9_block(const double* __restrict__ X, int64_t N, double* partials, int bx) {
+__device__ __forceinline__ void sum9_block(const double* X, int64_t N, double* partials, int bx) {
   __shared__ double red[9 * (CONST_THREADS / 32)];
   const int64_t v = int64_t(bx) * blockDim.x + threadIdx.x;
   double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -27,12 +27,20 @@ __device__ __forceinline__ void sum9_block(const double* __restrict__ X, int64_t
 #pragma unroll
     for (int k = 0; k < 9; ++k) partials[int64_t(bx) * 9 + k] = s[k];
 }
-__global__ void __launch_bounds__(CONST_THREADS) sum9_kernel(const double* __restrict__ X, int64_t N, double* partials) {
+__global__ void __launch_bounds__(CONST_THREADS) sum9_kernel(double* __restrict__ X, int64_t N, double* partials,
+                                                            const int* __restrict__ status,
+                                                            const double* __restrict__ kept) {
+  if (status && *status != 0) {
+    const int64_t v = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (v < N)
+#pragma unroll
+      for (int k = 0; k < 9; ++k) X[k * N + v] = kept[k * N + v];
+  }
   sum9_block(X, N, partials, blockIdx.x);
 }
-cudaError_t launch_sum9(const double* X, int64_t N, double* partials, cudaStream_t s) {
+cudaError_t launch_sum9(double* X, int64_t N, double* partials, cudaStream_t s, const int* status, const double* kept) {
   const int nb = int((N + CONST_THREADS - 1) / CONST_THREADS);
-  sum9_kernel<<<nb, CONST_THREADS, 0, s>>>(X, N, partials);
+  sum9_kernel<<<nb, CONST_THREADS, 0, s>>>(X, N, partials, status, kept);
   return cudaGetLastError();
 }
 

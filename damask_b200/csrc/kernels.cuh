@@ -83,6 +83,11 @@ template <int NS>
 cudaError_t launch_constitutive_begin(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f,
                                       const PassWork& w, double dt, int apply_update, BeginMode mode, int64_t v_begin,
                                       int64_t v_end, cudaStream_t s);
+// a whole evaluation in one launch, for grids of up to fused_voxels
+template <int NS>
+cudaError_t launch_constitutive_fused(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f, const PassWork& w,
+                                      double dt, int apply_update, int use_dot0, cudaStream_t s);
+int64_t fused_voxels(int ns, int nsm);
 // variant: the stress kernel's register bound (stress_variant_blocks: resident blocks per SM)
 template <int NS>
 cudaError_t launch_constitutive_pass(const PhaseConst<NS>& pc, const Numerics& nm, const Fields& f,
@@ -114,7 +119,10 @@ struct BatchPassBuffers {
 template <int NS>
 cudaError_t build_batch_pass_graph(const PhaseConst<NS>& pc, const Numerics& nm, const BatchTables& t,
                                    const BatchPassBuffers& b, int nsm, cudaStream_t s, cudaGraph_t* out);
-cudaError_t launch_sum9(const double* X, int64_t N, double* partials, cudaStream_t s);
+// block sums of the 9-plane field X; with status (device): where it is not 0, X := kept first (the
+// stress field is committed only when no voxel failed)
+cudaError_t launch_sum9(double* X, int64_t N, double* partials, cudaStream_t s, const int* status = nullptr,
+                        const double* kept = nullptr);
 cudaError_t launch_aim(SolverScalars* sc, const double* partials, int nparts, double wgt, int update_aim, cudaStream_t s);
 cudaError_t launch_converge(SolverScalars* sc, const double* div_partials, int nparts, double wgt, const int* status,
                             const Numerics2& nm2, int count_iteration, cudaStream_t s);
