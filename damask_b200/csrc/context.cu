@@ -855,7 +855,7 @@ int solution_polarization(dmk_ctx* c, dmk_solution_state* out) {
       const int mk = std::min(count, m);
       for (int q = count - mk; q < count; ++q) slots_b.push_back(q % m);
       nsl = int(slots_b.size());
-      CKL(launch_aa_dots(c->r, c->aa_Rprev, c->aa_dR, n18, new_slot, slots_b.data(), nsl, c->aa_partials, c->aa_blocks,
+      CKL(launch_aa_dots(c->r, c->aa_Rprev, c->aa_dX, c->aa_dR, n18, new_slot, true, slots_b.data(), nsl, c->aa_partials, c->aa_blocks,
                         c->aa_out, c->stream));
       c->launches += 2 * ((nsl + AA_CHUNK_HOST - 1) / AA_CHUNK_HOST) - 1;
       CK(cudaMemcpyAsync(dots, c->aa_out, sizeof(double) * 2 * AA_CHUNK_HOST * ((nsl + AA_CHUNK_HOST - 1) / AA_CHUNK_HOST),
@@ -933,7 +933,7 @@ int solution_polarization(dmk_ctx* c, dmk_solution_state* out) {
     } else {
       std::vector<double> gam = anderson_coefficients(G, m, slots_b, bvec);
       new_slot = count % m;
-      CKL(launch_aa_update(c->Fsol, c->r, c->aa_Rprev, c->aa_dX, c->aa_dR, n18, new_slot, slots_b.data(), gam.data(),
+      CKL(launch_aa_update(c->Fsol, c->r, c->aa_Rprev, c->aa_dX, n18, new_slot, slots_b.data(), gam.data(),
                           int(slots_b.size()), c->aa_blocks, c->stream));
       ++count;
     }
@@ -1365,7 +1365,7 @@ int dmk_mech_solution(dmk_ctx* c, dmk_solution_state* out) {
         const int mk = std::min(count, m);
         for (int q = count - mk; q < count; ++q) slots_b.push_back(q % m);
         nsl = int(slots_b.size());
-        CKL(launch_aa_dots(c->r, c->aa_Rprev, c->aa_dR, n9, new_slot, slots_b.data(), nsl, c->aa_partials,
+        CKL(launch_aa_dots(c->r, c->aa_Rprev, c->aa_dX, c->aa_dR, n9, new_slot, pass == 0, slots_b.data(), nsl, c->aa_partials,
                           c->aa_blocks, c->aa_out, c->stream));
         c->launches += 2 * ((nsl + AA_CHUNK_HOST - 1) / AA_CHUNK_HOST) - 1;   // dots + reduce per chunk
         CK(cudaMemcpyAsync(dots, c->aa_out, sizeof(double) * 2 * AA_CHUNK_HOST * ((nsl + AA_CHUNK_HOST - 1) / AA_CHUNK_HOST),
@@ -1409,7 +1409,7 @@ int dmk_mech_solution(dmk_ctx* c, dmk_solution_state* out) {
     } else {
       std::vector<double> gam = anderson_coefficients(G, m, slots_b, bvec);
       new_slot = count % m;
-      CKL(launch_aa_update(c->Fsol, c->r, c->aa_Rprev, c->aa_dX, c->aa_dR, n9, new_slot, slots_b.data(), gam.data(),
+      CKL(launch_aa_update(c->Fsol, c->r, c->aa_Rprev, c->aa_dX, n9, new_slot, slots_b.data(), gam.data(),
                           int(slots_b.size()), c->aa_blocks, c->stream));
       ++count;
       if ((rc = evaluate(0))) return rc;

@@ -768,29 +768,53 @@ namespace dmk {
 // ------------------------------------------------------------------ Anderson acceleration
 // After an evaluation with residual R: dR[slot] = R - Rprev (if write_slot >= 0), and the
 // inner products g_t = dR[slot].dR[t] and b_t = dR[t].R for up to AA_CHUNK history slots
-// per launch (per-block partial sums, reduced by the caller in block order).
-
+// per launch (per-block partial sums, reduced by the caller in block order).  The update reads dX[t] and
+// dR[t] only as dX[t] - dR[t], so dX[slot] becomes that difference here (first: it still holds the step;
+// in the correction pass of the mixed form, which repeats the products of one slot with another residual,
+// it holds the step less the first pass's dR[slot], in dR).  Bound by HBM: the loads of two elements are
+// issued before the first store (a store that the following loads might alias kept one element in flight).
 __device__ __forceinline__ void aa_dots_block(const double* __restrict__ R, const double* __restrict__ Rprev,
-                                              double* __restrict__ dR, int64_t n, int write_slot, const AASlots& sl,
-                                              double* __restrict__ partials, int bx, int nb, bool write) {
+                                              double* dX, double* dR, int64_t n, int write_slot, bool first,
+                                              const AASlots& sl, double* __restrict__ partials, int bx, int nb) {
   __shared__ double red[2 * AA_CHUNK][8];
   double g[AA_CHUNK], b[AA_CHUNK];
 #pragma unroll
   for (int q = 0; q < AA_CHUNK; ++q) { g[q] = 0.0; b[q] = 0.0; }
-#pragma unroll 2
-  for (int64_t e = int64_t(bx) * blockDim.x + threadIdx.x; e < n; e += int64_t(nb) * blockDim.x) {
-    const double r = R[e];
-    double dn = 0.0;
-    if (write_slot >= 0) {
-      dn = r - Rprev[e];
-      if (write) dR[int64_t(write_slot) * n + e] = dn;
+  double* const dRw = dR + int64_t(write_slot) * n;
+  double* const dXw = dX + int64_t(write_slot) * n;
+  constexpr int U = 2;
+  const int64_t stride = int64_t(nb) * blockDim.x;
+  for (int64_t e0 = int64_t(bx) * blockDim.x + threadIdx.x; e0 < n; e0 += U * stride) {
+    double r[U], dn[U], dx[U], d[U][AA_CHUNK];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t e = e0 + u * stride;
+      if (e < n) {
+        r[u] = R[e];
+        dn[u] = Rprev[e];
+        if (sl.write) dx[u] = first ? dXw[e] : dXw[e] + dRw[e];
+#pragma unroll
+        for (int q = 0; q < AA_CHUNK; ++q)
+          if (q < sl.n && sl.slot[q] != write_slot) d[u][q] = dR[int64_t(sl.slot[q]) * n + e];
+      }
     }
 #pragma unroll
-    for (int q = 0; q < AA_CHUNK; ++q) {
-      if (q < sl.n) {
-        const double d = (sl.slot[q] == write_slot) ? dn : dR[int64_t(sl.slot[q]) * n + e];
-        g[q] = fma(dn, d, g[q]);
-        b[q] = fma(d, r, b[q]);
+    for (int u = 0; u < U; ++u) {
+      const int64_t e = e0 + u * stride;
+      if (e < n) {
+        dn[u] = r[u] - dn[u];
+#pragma unroll
+        for (int q = 0; q < AA_CHUNK; ++q) {
+          if (q < sl.n) {
+            const double dd = sl.slot[q] == write_slot ? dn[u] : d[u][q];
+            g[q] = fma(dn[u], dd, g[q]);
+            b[q] = fma(dd, r[u], b[q]);
+          }
+        }
+        if (sl.write) {
+          dRw[e] = dn[u];
+          dXw[e] = dx[u] - dn[u];
+        }
       }
     }
   }
@@ -812,9 +836,9 @@ __device__ __forceinline__ void aa_dots_block(const double* __restrict__ R, cons
   }
 }
 __global__ void __launch_bounds__(256)
-aa_dots_kernel(const double* __restrict__ R, const double* __restrict__ Rprev, double* __restrict__ dR, int64_t n,
-               int write_slot, AASlots sl, double* __restrict__ partials) {
-  aa_dots_block(R, Rprev, dR, n, write_slot, sl, partials, blockIdx.x, gridDim.x, true);
+aa_dots_kernel(const double* __restrict__ R, const double* __restrict__ Rprev, double* dX, double* dR, int64_t n,
+               int write_slot, int first, AASlots sl, double* __restrict__ partials) {
+  aa_dots_block(R, Rprev, dX, dR, n, write_slot, first != 0, sl, partials, blockIdx.x, gridDim.x);
 }
 
 // 16 lanes per output, each summing every 16th block partial, then a fixed-order combine
@@ -837,18 +861,19 @@ __global__ void __launch_bounds__(256) aa_reduce_kernel(const double* __restrict
   aa_reduce_body(partials, nblocks, out);
 }
 
-cudaError_t launch_aa_dots(const double* R, const double* Rprev, double* dR, int64_t n, int write_slot,
-                           const int* slots, int nslots, double* partials, int nblocks, double* out, cudaStream_t s) {
+cudaError_t launch_aa_dots(const double* R, const double* Rprev, double* dX, double* dR, int64_t n, int write_slot,
+                           bool first, const int* slots, int nslots, double* partials, int nblocks, double* out,
+                           cudaStream_t s) {
   // out: for each chunk c, 2*AA_CHUNK doubles (g then b)
   int done = 0, chunk = 0;
   do {
     AASlots sl;
     sl.n = std::min(AA_CHUNK, nslots - done);
     for (int q = 0; q < AA_CHUNK; ++q) sl.slot[q] = q < sl.n ? slots[done + q] : 0;
-    // the first chunk writes dR[write_slot]; later chunks need dn for g, so they
-    // recompute it from R - Rprev without writing
-    const int ws = write_slot;
-    aa_dots_kernel<<<nblocks, 256, 0, s>>>(R, Rprev, dR, n, ws, sl, partials);
+    // the last chunk writes dR[write_slot] and dX[write_slot]; the others form dR[write_slot] from
+    // R - Rprev as it does
+    sl.write = done + sl.n >= nslots;
+    aa_dots_kernel<<<nblocks, 256, 0, s>>>(R, Rprev, dX, dR, n, write_slot, first ? 1 : 0, sl, partials);
     aa_reduce_kernel<<<1, 256, 0, s>>>(partials, nblocks, out + chunk * 2 * AA_CHUNK);
     done += sl.n;
     ++chunk;
@@ -856,36 +881,53 @@ cudaError_t launch_aa_dots(const double* R, const double* Rprev, double* dR, int
   return cudaGetLastError();
 }
 
-// X <- X - R - sum_t gamma_t (dX[t] - dR[t]);  dX[new_slot] = X_new - X_old;  Rprev = R
+// X <- X - R - sum_t gamma_t E[t], E[t] = dX[t] - dR[t] as aa_dots_block left it in dX;
+// dX[new_slot] = X_new - X_old;  Rprev = R
 __device__ __forceinline__ void aa_update_block(double* __restrict__ X, const double* __restrict__ R,
-                                                double* __restrict__ Rprev, double* __restrict__ dX,
-                                                const double* __restrict__ dR, int64_t n, int new_slot,
-                                                const AAUpdate& u, int bx, int nb) {
-#pragma unroll 2
-  for (int64_t e = int64_t(bx) * blockDim.x + threadIdx.x; e < n; e += int64_t(nb) * blockDim.x) {
-    const double x = X[e], r = R[e];
-    double xn = x - r;
-    for (int q = 0; q < u.n; ++q) {
-      const int64_t off = int64_t(u.slot[q]) * n + e;
-      xn = fma(-u.gamma[q], dX[off] - dR[off], xn);
+                                                double* __restrict__ Rprev, double* __restrict__ dX, int64_t n,
+                                                int new_slot, const AAUpdate& u, int bx, int nb) {
+  constexpr int U = 2;
+  const int64_t stride = int64_t(nb) * blockDim.x;
+  for (int64_t e0 = int64_t(bx) * blockDim.x + threadIdx.x; e0 < n; e0 += U * stride) {
+    double x[U], r[U], xn[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int64_t e = e0 + k * stride;
+      if (e < n) {
+        x[k] = X[e];
+        r[k] = R[e];
+        xn[k] = x[k] - r[k];
+      }
     }
-    dX[int64_t(new_slot) * n + e] = xn - x;
-    X[e] = xn;
-    Rprev[e] = r;
+#pragma unroll 4
+    for (int q = 0; q < u.n; ++q)
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        const int64_t e = e0 + k * stride;
+        if (e < n) xn[k] = fma(-u.gamma[q], dX[int64_t(u.slot[q]) * n + e], xn[k]);
+      }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int64_t e = e0 + k * stride;
+      if (e < n) {
+        dX[int64_t(new_slot) * n + e] = xn[k] - x[k];
+        X[e] = xn[k];
+        Rprev[e] = r[k];
+      }
+    }
   }
 }
 __global__ void __launch_bounds__(256)
 aa_update_kernel(double* __restrict__ X, const double* __restrict__ R, double* __restrict__ Rprev,
-                 double* __restrict__ dX, const double* __restrict__ dR, int64_t n, int new_slot,
-                 const __grid_constant__ AAUpdate u) {
-  aa_update_block(X, R, Rprev, dX, dR, n, new_slot, u, blockIdx.x, gridDim.x);
+                 double* __restrict__ dX, int64_t n, int new_slot, const __grid_constant__ AAUpdate u) {
+  aa_update_block(X, R, Rprev, dX, n, new_slot, u, blockIdx.x, gridDim.x);
 }
-cudaError_t launch_aa_update(double* X, const double* R, double* Rprev, double* dX, const double* dR, int64_t n,
+cudaError_t launch_aa_update(double* X, const double* R, double* Rprev, double* dX, int64_t n,
                              int new_slot, const int* slots, const double* gamma, int nslots, int nblocks, cudaStream_t s) {
   AAUpdate u;
   u.n = nslots;
   for (int q = 0; q < 32; ++q) { u.slot[q] = q < nslots ? slots[q] : 0; u.gamma[q] = q < nslots ? gamma[q] : 0.0; }
-  aa_update_kernel<<<nblocks, 256, 0, s>>>(X, R, Rprev, dX, dR, n, new_slot, u);
+  aa_update_kernel<<<nblocks, 256, 0, s>>>(X, R, Rprev, dX, n, new_slot, u);
   return cudaGetLastError();
 }
 
@@ -1004,7 +1046,9 @@ __global__ void __launch_bounds__(256) batch_aa_dots_kernel(const BatchCtx* __re
   sl.n = min(AA_CHUNK, c.nsl - chunk * AA_CHUNK);
 #pragma unroll
   for (int q = 0; q < AA_CHUNK; ++q) sl.slot[q] = q < sl.n ? c.slots[chunk * AA_CHUNK + q] : 0;
-  aa_dots_block(c.r, c.Rprev, c.dR, 9 * c.N, c.write_slot, sl, c.aa_partials, blockIdx.x, c.aa_blocks, true);
+  sl.write = (chunk + 1) * AA_CHUNK >= c.nsl;
+  aa_dots_block(c.r, c.Rprev, c.dX, c.dR, 9 * c.N, c.write_slot, c.count_iter != 0, sl, c.aa_partials, blockIdx.x,
+                c.aa_blocks);
 }
 __global__ void __launch_bounds__(256) batch_aa_reduce_kernel(const BatchCtx* __restrict__ t, int chunk) {
   const BatchCtx& c = t[blockIdx.x];
@@ -1023,7 +1067,7 @@ __global__ void __launch_bounds__(256) batch_aa_update_kernel(const BatchCtx* __
   const BatchCtx& c = t[blockIdx.y];
   const BatchAA& a = u[blockIdx.y];
   if (!a.active || int(blockIdx.x) >= c.aa_blocks) return;
-  aa_update_block(c.X, c.r, c.Rprev, c.dX, c.dR, 9 * c.N, a.new_slot, a.u, blockIdx.x, c.aa_blocks);
+  aa_update_block(c.X, c.r, c.Rprev, c.dX, 9 * c.N, a.new_slot, a.u, blockIdx.x, c.aa_blocks);
 }
 cudaError_t launch_batch_aa_update(const BatchCtx* t, const BatchAA* u, int n_ctx, int max_blocks, cudaStream_t s) {
   if (n_ctx <= 0) return cudaSuccess;

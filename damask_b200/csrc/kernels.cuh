@@ -179,16 +179,18 @@ constexpr int AA_CHUNK = 8;    // history slots per inner-product launch
 struct AASlots {
   int n;                       // slots in this chunk
   int slot[AA_CHUNK];
+  int write;                   // this launch writes dR and dX of the new slot
 };
 struct AAUpdate {              // X <- X - R - sum_q gamma_q (dX[slot_q] - dR[slot_q])
   int n;
   int slot[AA_MAX];
   double gamma[AA_MAX];
 };
-cudaError_t launch_aa_dots(const double* R, const double* Rprev, double* dR, int64_t n, int write_slot,
-                           const int* slots, int nslots, double* partials, int nblocks, double* out, cudaStream_t s);
-cudaError_t launch_aa_update(double* X, const double* R, double* Rprev, double* dX, const double* dR, int64_t n,
-                             int new_slot, const int* slots, const double* gamma, int nslots, int nblocks, cudaStream_t s);
+cudaError_t launch_aa_dots(const double* R, const double* Rprev, double* dX, double* dR, int64_t n, int write_slot,
+                           bool first, const int* slots, int nslots, double* partials, int nblocks, double* out,
+                           cudaStream_t s);
+cudaError_t launch_aa_update(double* X, const double* R, double* Rprev, double* dX, int64_t n, int new_slot,
+                             const int* slots, const double* gamma, int nslots, int nblocks, cudaStream_t s);
 
 // ------------------------------------------------------------------ batches of contexts (kernels.cu)
 // The fixed-point iteration of many contexts (RVEs) in shared launches.  Each context is one entry
