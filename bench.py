@@ -36,13 +36,13 @@ FP64_NOMINAL_TFLOPS = 37.0   # B200 FP64 (CUDA cores), datasheet figure
 
 
 def constitutive_flops(ns: int, newton: float, state: float, updates: float) -> float:
-    """Static FP64 FLOP count of the constitutive passes (FMA = 2):
-    per residual evaluation (Newton iteration) 264 + 56 Ns; per Newton step (Woodbury
-    6x6 system: assembly, QR, back-substitution; one per non-final Newton iteration)
-    567 + 135 Ns; per state iteration (stress start/finish, hardening, damped update)
-    455 + 86 Ns; per substep start (kinetics and hardening) 89 Ns."""
+    """Static FP64 FLOP count of the constitutive passes for a phase without non-Schmid terms
+    (FMA = 2): per residual evaluation (Newton iteration) 173 + 40 Ns; per Newton step (the
+    five-unknown system: assembly, QR, back-substitution; one per non-final Newton iteration)
+    800 + 65 Ns; per state iteration (stress start/finish, hardening, damped update)
+    410 + 86 Ns; per substep start (kinetics and hardening) 89 Ns."""
     steps = max(newton - state, 0.0)
-    return newton * (264 + 56 * ns) + steps * (567 + 135 * ns) + state * (455 + 86 * ns) + updates * (89 * ns)
+    return newton * (173 + 40 * ns) + steps * (800 + 65 * ns) + state * (410 + 86 * ns) + updates * (89 * ns)
 
 
 # DRAM bytes that one stress and one control launch move per voxel of a full pass, by slip-system
