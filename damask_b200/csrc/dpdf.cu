@@ -273,29 +273,39 @@ dPdF_kernel(const __grid_constant__ PhaseConst<NS> pc, const __grid_constant__ F
 // of that range (fixed summation order).
 constexpr int TSUM_THREADS = 256, TSUM_BLOCKS = 1184;
 
+// grid.y: nine components of the 81 each, summed together; one block for all of them was 81 reductions one
+// after the other, each a memory round trip and two barriers (45 us whatever the size, 154 us at 64^3).  The
+// sums keep their order.
+constexpr int TSUM_COMPONENTS = 9;
 __global__ void __launch_bounds__(TSUM_THREADS)
 tangent_sum_kernel(const double* __restrict__ planes, const double* __restrict__ norms, int64_t first, int64_t count,
                    int64_t N, TangentOut o) {
-  __shared__ double red[TSUM_THREADS / 32];
+  __shared__ double red[TSUM_COMPONENTS][TSUM_THREADS / 32];
   __shared__ double rmax[TSUM_THREADS / 32], rmin[TSUM_THREADS / 32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int c0 = blockIdx.y * TSUM_COMPONENTS;
   const int64_t per = (count + gridDim.x - 1) / gridDim.x;
   const int64_t b0 = first + int64_t(blockIdx.x) * per;
   const int64_t b1 = b0 + per < first + count ? b0 + per : first + count;
-  for (int c = 0; c < 81; ++c) {
-    double s = 0.0;
-    for (int64_t v = b0 + t; v < b1; v += TSUM_THREADS) s += planes[int64_t(c) * N + v];
+  double s[TSUM_COMPONENTS];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if (lane == 0) red[w] = s;
-    __syncthreads();
-    if (t == 0) {
-      double tot = 0.0;
-      for (int k = 0; k < TSUM_THREADS / 32; ++k) tot += red[k];
-      o.partials[int64_t(blockIdx.x) * 81 + c] = tot;
-    }
-    __syncthreads();
+  for (int k = 0; k < TSUM_COMPONENTS; ++k) s[k] = 0.0;
+  for (int64_t v = b0 + t; v < b1; v += TSUM_THREADS)
+#pragma unroll
+    for (int k = 0; k < TSUM_COMPONENTS; ++k) s[k] += planes[int64_t(c0 + k) * N + v];
+#pragma unroll
+  for (int k = 0; k < TSUM_COMPONENTS; ++k) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], off);
+    if (lane == 0) red[k][w] = s[k];
   }
+  __syncthreads();
+  if (t < TSUM_COMPONENTS) {
+    double tot = 0.0;
+    for (int k = 0; k < TSUM_THREADS / 32; ++k) tot += red[t][k];
+    o.partials[int64_t(blockIdx.x) * 81 + c0 + t] = tot;
+  }
+  if (blockIdx.y != 0) return;
   double mx = 0.0, mn = 1.7976931348623157e308;
   for (int64_t v = b0 + t; v < b1; v += TSUM_THREADS) {
     mx = fmax(mx, norms[v]);
@@ -354,12 +364,12 @@ cudaError_t launch_dPdF(const PhaseConst<NS>& pc, const Fields& f, double dt, co
   if (e != cudaSuccess) return e;
   const int nb = int((count + TAN_THREADS - 1) / TAN_THREADS);
   dPdF_kernel<NS><<<nb, TAN_THREADS, smem, s>>>(pc, f, dt, o, first, count);
-  if (with_sums) tangent_sum_kernel<<<dPdF_blocks(count), TSUM_THREADS, 0, s>>>(o.planes, o.norms, first, count, f.N, o);
+  if (with_sums) tangent_sum_kernel<<<dim3(dPdF_blocks(count), 81 / TSUM_COMPONENTS), TSUM_THREADS, 0, s>>>(o.planes, o.norms, first, count, f.N, o);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tangent_sums(const TangentOut& o, int64_t first, int64_t count, int64_t N, cudaStream_t s) {
-  tangent_sum_kernel<<<dPdF_blocks(count), TSUM_THREADS, 0, s>>>(o.planes, o.norms, first, count, N, o);
+  tangent_sum_kernel<<<dim3(dPdF_blocks(count), 81 / TSUM_COMPONENTS), TSUM_THREADS, 0, s>>>(o.planes, o.norms, first, count, N, o);
   return cudaGetLastError();
 }
 template cudaError_t launch_dPdF<12>(const PhaseConst<12>&, const Fields&, double, const TangentOut&, int64_t, int64_t,

@@ -74,22 +74,29 @@ __device__ void rot33(const double* qin, const double* T, double* R, bool active
 // After the constitutive sweep: P_av = <P> (rotated to the load frame),
 // deltaF_aim = S : (P_av - P_aim), F_aim -= deltaF_aim, err_BC, and the rotated
 // aim for the DC term of the Gamma convolution (form_residual, grid_mech_spectral_basic.f90:503-519).
+// A warp per component of P (AIM_THREADS), each lane its share of the blocks with several loads in
+// flight: one warp for all nine was a chain of dependent loads (131 us at 16384 partial sums, 128^3).  The
+// sums keep their order.
+constexpr int AIM_THREADS = 9 * 32;
 __device__ __forceinline__ void aim_body(SolverScalars* sc, const double* partials, int nparts, double wgt, int update_aim) {
   __shared__ double acc[9][32];
+  __shared__ double Pav[9];
   const int t = threadIdx.x;
-  for (int k = 0; k < 9; ++k) {
+  {
+    const int k = t >> 5, lane = t & 31;
     double s = 0.0;
-    for (int b = t; b < nparts; b += 32) s += partials[int64_t(b) * 9 + k];
-    acc[k][t] = s;
+#pragma unroll 8
+    for (int b = lane; b < nparts; b += 32) s += partials[int64_t(b) * 9 + k];
+    acc[k][lane] = s;
   }
-  __syncwarp();
+  __syncthreads();
+  if (t < 9) {
+    double s = 0.0;
+    for (int w = 0; w < 32; ++w) s += acc[t][w];
+    Pav[t] = s * wgt;
+  }
+  __syncthreads();
   if (t != 0) return;
-  double Pav[9];
-  for (int k = 0; k < 9; ++k) {
-    double s = 0.0;
-    for (int w = 0; w < 32; ++w) s += acc[k][w];
-    Pav[k] = s * wgt;
-  }
   double R[9];
   rot33(sc->q_rot, Pav, R, false);
   for (int k = 0; k < 9; ++k) sc->P_av[k] = R[k];
@@ -123,6 +130,7 @@ __device__ __forceinline__ void converge_body(SolverScalars* sc, const double* d
   __shared__ double acc[32];
   const int t = threadIdx.x;
   double s = 0.0;
+#pragma unroll 8
   for (int b = t; b < nparts; b += 32) s += div_partials[b];
   acc[t] = s;
   __syncwarp();
@@ -152,7 +160,7 @@ __global__ void converge_kernel(SolverScalars* sc, const double* div_partials, i
 }
 
 cudaError_t launch_aim(SolverScalars* sc, const double* partials, int nparts, double wgt, int update_aim, cudaStream_t s) {
-  aim_kernel<<<1, 32, 0, s>>>(sc, partials, nparts, wgt, update_aim);
+  aim_kernel<<<1, AIM_THREADS, 0, s>>>(sc, partials, nparts, wgt, update_aim);
   return cudaGetLastError();
 }
 cudaError_t launch_converge(SolverScalars* sc, const double* div_partials, int nparts, double wgt, const int* status,
@@ -948,7 +956,7 @@ __global__ void batch_aim_kernel(const BatchCtx* __restrict__ t) {
 cudaError_t launch_batch_aim(const BatchCtx* t, int n_ctx, int max_nconst, cudaStream_t s) {
   if (n_ctx <= 0) return cudaSuccess;
   batch_sum9_kernel<<<dim3(max_nconst, n_ctx), CONST_THREADS, 0, s>>>(t);
-  batch_aim_kernel<<<n_ctx, 32, 0, s>>>(t);
+  batch_aim_kernel<<<n_ctx, AIM_THREADS, 0, s>>>(t);
   return cudaGetLastError();
 }
 
