@@ -46,11 +46,12 @@ def constitutive_flops(ns: int, newton: float, state: float, updates: float) -> 
 
 
 # DRAM bytes that one stress and one control launch move per voxel of a full pass, by slip-system
-# count, from the ncu captures summarised in profiles/constitutive_passes_64cubed_bcc24.txt and
-# _bcc48.txt (two passes of a 65 536-voxel chunk each; 24 systems: stress 568 B, control 2 114 B;
-# 48 systems: stress 794 B, control 4 840 B); a material-point update runs one such pass per state
-# iteration
-TRAFFIC_BYTES_PER_PASS = {24: 2682, 48: 5634}
+# count, from the ncu captures summarised in profiles/constitutive_passes_96x96x64_bcc24.txt (24
+# systems: mean of the first pass, stress 1.11 kB and control 1.77 kB, and the second, 0.92 and 2.61 kB)
+# and profiles/constitutive_passes_64cubed_bcc48.txt (48 systems, before the start state of an
+# evaluation was no longer stored: stress 794 B, control 4 840 B); a material-point update runs one such
+# pass per state iteration
+TRAFFIC_BYTES_PER_PASS = {24: 3205, 48: 5634}
 
 # the 48-system RVE's window inside the default bench line (5.7 s per increment at 256^3)
 BCC48_WARMUP, BCC48_STEPS = 3, 3
@@ -519,7 +520,8 @@ def measure(workload, steps, warmup, world, rank, local, cells, solver, derivati
         'flops_per_update': flops / max(1, mx['updates']),
         'flop_source': 'static FP64 count of the kernels times the counted Newton / state iterations',
         'traffic': traffic * mx['N'] if traffic else None,
-        'traffic_source': f'ncu DRAM bytes of a stress and a control launch per voxel and pass at 64^3 ({ns} systems), '
+        'traffic_source': f'ncu DRAM bytes of a stress and a control launch per voxel and pass ({ns} systems; 24: mean of the '
+                          'first two passes at 96x96x64, 48: at 64^3 with the start state still stored), '
                           'times the passes (state iterations) per update and the voxels of one evaluation; '
                           'the begin kernel is not included',
         'avg_launch_ms': avg_launch_ms,
