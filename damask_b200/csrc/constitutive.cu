@@ -337,7 +337,9 @@ constitutive_control_kernel(const __grid_constant__ PhaseConst<NS> pc, const __g
 // One evaluation of a small grid in one launch: every voxel's begin, and its stress integrations and
 // control steps one after the other until it is done.  No voxel lists and no host between passes.  With
 // every voxel resident at once there is nothing that the lists' compaction could gain, and what
-// bounds such a grid is the chain of one voxel, launches and host round trips.
+// bounds such a grid is the chain of one voxel, launches and host round trips.  The loop ends after
+// max_passes stress integrations as the pass loop of larger grids does: control flow alone does not
+// (a failing voxel with r_cutback >= 1 starts the same substep again without end).
 template <int NS, bool SCHMID>
 struct FusedShape : StressShape<NS, SCHMID, 2> {
   using Base = StressShape<NS, SCHMID, 2>;
@@ -365,6 +367,10 @@ constitutive_fused_kernel(const __grid_constant__ PhaseConst<NS> pc, const __gri
   int nstate = 0, newton = 0;
   bool keep = v < f.N && begin_voxel<NS>(pc, hs, xs, nm, f, w, v, dt, apply_update, use_dot0);
   while (keep) {
+    if (nstate >= nm.max_passes) {
+      atomicMax(f.status, STATUS_PASS_LIMIT);
+      break;
+    }
     newton += stress_voxel<NS, Shape>(pc, sc, xs, nm, f, w, v, dt);
     ++nstate;
     keep = control_voxel<NS>(pc, hs, xs, nm, f, w, v, dt);

@@ -217,6 +217,8 @@ PassWork pass_work(dmk_ctx* c, int half, int out) {
 }
 size_t pass_work_doubles(int64_t N, int NS) { return size_t(N) * size_t(36 + 7 * NS + 2); }
 
+int pass_limit_error() { return fail(DMK_ERR_CUDA, "constitutive passes did not terminate"); }
+
 template <int NS>
 int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, double dt, int apply) {
   if (c->N <= fused_voxels(NS, c->nsm)) {
@@ -236,7 +238,7 @@ int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, d
   // the other streams start after everything queued on the first
   CK(cudaEventRecord(c->fork, c->stream));
   for (int h = 1; h < K; ++h) CK(cudaStreamWaitEvent(c->cstream[h], c->fork, 0));
-  int cur[PASS_CHUNKS];
+  int cur[PASS_CHUNKS], done[PASS_CHUNKS] = {};
   bool active[PASS_CHUNKS];
   for (int h = 0; h < K; ++h) {
     // pass 0: restore and control up to the first integrateStress of every voxel of the chunk
@@ -249,7 +251,7 @@ int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, d
   }
   c->dot0_valid = true;   // the begin kernels above stored (or read) the increment-start rates
   // each chunk advances as soon as its previous pass has ended, so the chunks pipeline
-  for (int pass = 1;;) {
+  for (;;) {
     bool any = false;
     for (int h = 0; h < K; ++h) {
       if (!active[h]) continue;
@@ -257,8 +259,10 @@ int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, d
       const int64_t n = c->hcount[h];
       if (n == 0) { active[h] = false; continue; }
       any = true;
-      // bounded by substeps x state iterations; a runaway count means corrupted control state
-      if (++pass > 400000) return fail(DMK_ERR_CUDA, "constitutive passes did not terminate");
+      if (++done[h] > c->nm.max_passes) {
+        for (int k = 0; k < K; ++k) CK(cudaStreamSynchronize(c->cstream[k]));
+        return pass_limit_error();
+      }
       const int nxt = 1 - cur[h];
       CK(cudaMemsetAsync(c->pcount + 2 * h + nxt, 0, sizeof(int), c->cstream[h]));
       CKL(launch_constitutive_pass<NS>(pc, c->nm, f, pass_work(c, h, nxt), dt, c->plist[h][cur[h]], n,
@@ -563,6 +567,8 @@ int enqueue_constitutive(dmk_ctx* c, double dt, const double* r, int apply, cons
   CKL(launch_sum9(c->P, c->N, c->partials, c->stream, c->status, c->Pnew));   // <P> of the committed stress field
   return 0;
 }
+// the error of a sweep that stopped at the limit of its passes (pass lists report it at once)
+int check_pass_limit(int status) { return status == STATUS_PASS_LIMIT ? pass_limit_error() : 0; }
 // the time of the last sweep, once the stream has passed it
 int add_constitutive_ms(dmk_ctx* c) {
   float ms = 0.f;
@@ -577,6 +583,7 @@ int evaluate_constitutive(dmk_ctx* c, double dt, const double* r, int apply, int
   CK(cudaMemcpyAsync(c->hcount, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   *status_out = c->hcount[0];
+  if (int rc = check_pass_limit(*status_out)) return rc;
   return add_constitutive_ms(c);
 }
 
@@ -1090,6 +1097,7 @@ int dmk_mech_init(dmk_ctx** out, const int cells[3], const double geomSize[3], c
   c->nm.eps_rel_state = num->eps_rel_state; c->nm.N_iter_state_max = num->N_iter_state_max;
   c->nm.N_iter_Lp_max = num->N_iter_Lp_max; c->nm.r_linesearch_Lp = num->r_linesearch_Lp;
   c->nm.eps_rel_Lp = num->eps_rel_Lp; c->nm.eps_abs_Lp = num->eps_abs_Lp; c->nm.f_update_jacobi_Lp = num->f_update_jacobi_Lp;
+  c->nm.max_passes = MAX_PASSES;
   c->nm2.N_iter_min = num->N_iter_min; c->nm2.N_iter_max = num->N_iter_max; c->nm2.cells0 = cells[0];
   c->nm2.eps_abs_div = num->eps_abs_div; c->nm2.eps_rel_div = num->eps_rel_div;
   c->nm2.eps_abs_P = num->eps_abs_P; c->nm2.eps_rel_P = num->eps_rel_P;
@@ -1376,6 +1384,7 @@ int dmk_mech_solution(dmk_ctx* c, dmk_solution_state* out) {
       float ms = 0.f;
       CK(cudaEventElapsedTime(&ms, c->ev[2], c->ev[3]));
       c->last_ms[1] += ms;
+      if (int e = check_pass_limit(hs.status)) return e;
       if (pass == 0)
         if (int e = add_constitutive_ms(c)) return e;
       if (nsl > 0) {
@@ -2524,7 +2533,7 @@ int batch_build(dmk_batch* b) {
   pb.status = b->d_status;
   pb.n_ctx = n;
   pb.iter = b->d_iter;
-  pb.max_passes = 400000;   // bounded by substeps x state iterations; more means corrupted control state
+  pb.max_passes = b->ctx[0]->nm.max_passes;
   cudaError_t e = cudaErrorInvalidValue;
   switch (b->NS) {
     case 12: e = batch_graph<12>(b, t, pb); break;
@@ -2678,7 +2687,7 @@ int batch_solution_impl(dmk_batch* b, const int* which, int nw, dmk_solution_sta
     CK(cudaEventElapsedTime(&ms, b->ev[2], b->ev[3]));
     b->last_ms[0] += ms;
     b->passes += b->h_iter[0];
-    if (b->h_iter[1]) return fail(DMK_ERR_CUDA, "constitutive passes did not terminate");
+    if (b->h_iter[1]) return pass_limit_error();
     // FP32 passes that meet the tolerance get a correction pass in FP64 on the same stress field;
     // its residual, decision and inner products replace the FP32 ones (dmk_mech_solution's)
     int ncorr = 0, nch1 = 0;
@@ -2943,6 +2952,13 @@ int dmk_get_tuning(dmk_ctx* c, int* stress_blocks, int* chunks) {
   if (!c) return fail(DMK_ERR_ARG, "null argument");
   if (stress_blocks) *stress_blocks = stress_variant_blocks(c->NS, c->stress_variant);
   if (chunks) *chunks = c->nchunks;
+  return 0;
+}
+
+int dmk_set_pass_limit(dmk_ctx* c, int limit) {
+  if (!c) return fail(DMK_ERR_ARG, "null argument");
+  if (limit < 1) return fail(DMK_ERR_ARG, "the limit of the constitutive passes must be positive");
+  c->nm.max_passes = limit;
   return 0;
 }
 

@@ -47,6 +47,7 @@ struct Numerics {
   int N_iter_state_max, N_iter_Lp_max;
   double r_linesearch_Lp, eps_rel_Lp, eps_abs_Lp;
   int f_update_jacobi_Lp;
+  int max_passes;        // stress integrations of a voxel in one evaluation; more are an error
 };
 
 // Device pointers of one RVE's fields.
@@ -67,7 +68,7 @@ struct Fields {
   double* state;    // (2 NS)
   double* state0;   // (2 NS)
   double* partials; // per block: 9 sums of P
-  int* status;      // worst status (atomicMax)
+  int* status;      // worst status (atomicMax): 2 a voxel failed, STATUS_PASS_LIMIT
   int* iter;        // optional per-voxel counters: 4 ints per voxel (planes)
   unsigned long long* counters;   // [0] evaluations [1] state iterations [2] Newton iterations
 };
@@ -96,6 +97,10 @@ struct PassWork {
 };
 
 enum : int { PH_CTRL = 0, PH_DOT0 = 1, PH_STRESS = 2, PH_DOT1 = 3, PH_DONE = 4 };
+
+// status of an evaluation in which a voxel needed more than Numerics::max_passes stress integrations; the
+// host turns it into an error
+constexpr int STATUS_PASS_LIMIT = 100;
 
 // from_start: the running state iteration started from the increment-start state and rate (the first
 // attempt of the first substep); it is kept as the sign of the stored step.  Its start state, state0 +

@@ -5,6 +5,7 @@
 namespace dmk {
 
 constexpr int CONST_THREADS = 128;   // block size of the per-voxel partial sums of P
+constexpr int MAX_PASSES = 400000;   // default of Numerics::max_passes
 constexpr int PASS_CHUNKS = 4;       // voxel chunks whose constitutive passes run on their own streams
 constexpr int SPEC_THREADS = 256;    // spectral pointwise kernels
 

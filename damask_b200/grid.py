@@ -124,6 +124,10 @@ class SpectralBasic:
     def set_tuning(self, stress_blocks: int, chunks: int) -> None:
         _lib.check(self.lib.dmk_set_tuning(self.ctx, int(stress_blocks), int(chunks)))
 
+    def set_pass_limit(self, limit: int) -> None:
+        """Most stress integrations of a voxel in one constitutive evaluation (dmk_set_pass_limit)."""
+        _lib.check(self.lib.dmk_set_pass_limit(self.ctx, int(limit)))
+
     def update_coords(self) -> None:
         _lib.check(self.lib.dmk_mech_update_coords(self.ctx))
 

@@ -331,6 +331,12 @@ int dmk_autotune(dmk_ctx* ctx, int reps, double* report, int* n_report);
 int dmk_get_tuning(dmk_ctx* ctx, int* stress_blocks, int* chunks);
 int dmk_set_tuning(dmk_ctx* ctx, int stress_blocks, int chunks);
 
+/* Limit of the stress integrations of a voxel in one constitutive evaluation (default 400000), whatever
+   form the evaluation takes: a voxel that needs more ends it with DMK_ERR_CUDA ("constitutive passes
+   did not terminate").  Numerics with r_cutback >= 1 can ask for any number of them.  A batch takes the
+   limit that its contexts have when it is created. */
+int dmk_set_pass_limit(dmk_ctx* ctx, int limit);
+
 /* Number of kernels of this library launched by the context so far. */
 int dmk_get_launches(dmk_ctx* ctx, int64_t* out);
 /* Device timer on the context's stream: CUDA events recorded at start and stop;
