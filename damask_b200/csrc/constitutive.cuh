@@ -746,7 +746,14 @@ __device__ void advance(const PhaseConst<NS>& pc, const double* __restrict__ hs,
         c.phase = PH_STRESS;
       } else {
         // integrateStateFPI:631-646 (the stress integration of this iteration succeeded: status 0)
-        if (bad) { c.phase = PH_CTRL; continue; }
+        if (bad) {
+          // the state stays what this iteration started from, which a fresh start has not stored
+          if (fresh)
+#pragma unroll 1
+            for (int i = 0; i < NST; ++i) f.state[i * N + v] = state(i);
+          c.phase = PH_CTRL;
+          continue;
+        }
         // generations: dotState of the last iteration (it - 1) and the one before (it - 2,
         // whose storage receives the damped rate of this iteration)
         const double* L1 = fresh ? w.dot0 + v : dot_gen(w, c.it + 1, NST, N) + v;

@@ -89,6 +89,35 @@ def test_failure_status_matches(gpu, oracle_lib):
     g.close()
 
 
+@pytest.mark.parametrize('cells', [(2, 3, 2), (64, 37, 17)])          # one launch, voxel lists
+def test_state_after_a_nan_rate(gpu, oracle_lib, cells):
+    """Saturated slip (xi_0 = xi_inf, a power of two: 1 - xi/xi_inf is exactly zero) with interactions so large
+    that the hardening sum overflows at high rates makes a state rate 0 * inf = NaN after a converged
+    stress integration.  The state iteration ends there, with the state that it started from and not what
+    an earlier evaluation of the increment left."""
+    phase = workloads.fcc_al(xi_0=2.0**25, xi_inf=2.0**25)
+    phase.h_sl_sl = [1.0e308] * 7
+    # few different voxels: the oracle sweeps a small grid of the same ones
+    n, few = int(np.prod(cells)), 12
+    q = np.random.default_rng(3).normal(size=(few, 4))
+    q *= np.sign(q[:, :1]) / np.linalg.norm(q, axis=1, keepdims=True)
+    g = SpectralBasic(cells, workloads.SIZE_1MM, np.arange(n) % few, q, phase, workloads.numerics_default())
+    o = oracle_lib.OracleSpectralBasic((few, 1, 1), workloads.SIZE_1MM, np.arange(few), q, phase,
+                                       workloads.numerics_default(), threads=4)
+    F = (np.eye(3) + np.diag([2e-3, -8e-4, -8e-4])).reshape(-1)
+    for dt in (1.0, 1e-10):
+        sg = g.constitutive_response(np.tile(F, (n, 1)), dt)[-1]
+        so = o.constitutive_response(np.tile(F, (few, 1)), dt)[-1]
+        assert sg == so == 0
+        for name in ('xi_sl', 'gamma_sl', 'L_p', 'F_p', 'S'):
+            a, b = g.get_field(name), o.get_field(name)[np.arange(n) % few]
+            assert np.isfinite(b).all() and rel(a, b) < TOL, (dt, name)
+        if dt == 1.0:
+            assert g.get_field('gamma_sl').max() > 1e-5               # the first evaluation left slip
+    assert np.all(g.get_field('gamma_sl') == 0.0)                     # the increment started from none
+    g.close()
+
+
 def test_spectral_operators(gpu, oracle_lib, golden):
     num = workloads.numerics_default()
     num.divergence_correction = 'size'
