@@ -217,11 +217,14 @@ PassWork pass_work(dmk_ctx* c, int half, int out) {
 }
 size_t pass_work_doubles(int64_t N, int NS) { return size_t(N) * size_t(36 + 7 * NS + 2); }
 
+// evaluations of the context run as one launch instead of passes over voxel lists
+bool one_launch(const dmk_ctx* c) { return c->N <= fused_voxels(c->NS, c->nsm); }
+
 int pass_limit_error() { return fail(DMK_ERR_CUDA, "constitutive passes did not terminate"); }
 
 template <int NS>
 int constitutive_passes(dmk_ctx* c, const PhaseConst<NS>& pc, const Fields& f, double dt, int apply) {
-  if (c->N <= fused_voxels(NS, c->nsm)) {
+  if (one_launch(c)) {
     CKL(launch_constitutive_fused<NS>(pc, c->nm, f, pass_work(c, 0, 0), dt, apply, c->dot0_valid ? 1 : 0, c->stream));
     ++c->passes;
     c->dot0_valid = true;
@@ -2863,7 +2866,8 @@ dmk_ctx* batch_member(dmk_batch* b, int k) { return (b && k >= 0 && k < b->n) ? 
 // slip systems) and voxel-chunk count (1, 2, 4); the fastest pair is kept.  The fields an
 // evaluation changes (Fp, Lp, S, Fe, state) are copied to a scratch buffer first and restored after
 // every trial, and the stress buffers are swapped back, so a solve after the tuning runs bit for bit
-// as without it (the variants and chunk counts change the schedule, not the arithmetic).
+// as without it (the variants and chunk counts change the schedule, not the arithmetic).  Grids whose
+// evaluations run as one launch use neither variants nor chunks: nothing is timed or changed there.
 
 namespace {
 
@@ -2883,6 +2887,10 @@ int copy_buffers(dmk_ctx* c, double* scratch, bool save) {
 }
 
 int autotune_impl(dmk_ctx* c, int reps, double* report, int* n_report) {
+  if (one_launch(c)) {
+    if (n_report) *n_report = 0;
+    return 0;
+  }
   size_t total = 0;
   for (const auto& b : tuning_buffers(c)) total += b.second;
   size_t free_b = 0, total_b = 0;

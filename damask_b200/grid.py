@@ -108,7 +108,8 @@ class SpectralBasic:
 
     def autotune(self, reps: int = 2) -> dict:
         """dmk_autotune: time the constitutive evaluation at the current state for every stress-kernel
-        variant and voxel-chunk count and keep the fastest (results unchanged)."""
+        variant and voxel-chunk count and keep the fastest (results unchanged).  No candidates, and nothing
+        changed, on a small grid whose evaluations run as one launch."""
         rep = np.zeros(36)
         n = C.c_int()
         _lib.check(self.lib.dmk_autotune(self.ctx, int(reps), _dp(rep), C.byref(n)))

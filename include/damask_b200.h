@@ -326,7 +326,10 @@ int dmk_fp64_peak(int device, double* tflops);
    keeps the fastest pair.  The fields an evaluation changes are restored after every trial, so the
    solve continues bit for bit as without tuning.  Needs free device memory for a copy of Fp, Lp, S,
    Fe and the state (fails with DMK_ERR_CUDA otherwise, leaving the settings).  report (optional, 36
-   doubles): per candidate (blocks per SM, chunks, ms); *n_report candidates.  Basic scheme only. */
+   doubles): per candidate (blocks per SM, chunks, ms); *n_report candidates.  Basic scheme only.
+   Grids of up to 256 voxels per SM (128 at 48 systems) run an evaluation as one launch, without
+   variants or chunks: dmk_autotune then times nothing, keeps the settings and reports no candidates,
+   and dmk_set_tuning has no effect.  The one variant at 48 systems is named 1. */
 int dmk_autotune(dmk_ctx* ctx, int reps, double* report, int* n_report);
 int dmk_get_tuning(dmk_ctx* ctx, int* stress_blocks, int* chunks);
 int dmk_set_tuning(dmk_ctx* ctx, int stress_blocks, int chunks);

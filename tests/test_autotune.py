@@ -8,9 +8,12 @@ from damask_b200.grid import IncrementDriver, SpectralBasic
 
 pytestmark = pytest.mark.gpu
 
+LISTS = (48, 32, 32)       # evaluated by passes over voxel lists, which the variants and chunks belong to
+ONE_LAUNCH = (32, 32, 32)
 
-def _run(tune_at, n=4):
-    rve, phase, lcs, num = workloads.make_cut('grid256_bcc24_2000g', (32, 32, 32))
+
+def _run(tune_at, n=4, cells=LISTS):
+    rve, phase, lcs, num = workloads.make_cut('grid256_bcc24_2000g', cells)
     s = SpectralBasic(rve.cells, rve.size, rve.material, rve.quaternions, phase, num)
     drv = IncrementDriver(s, lcs)
     stats, tuning = [], None
@@ -43,6 +46,21 @@ def test_autotune_keeps_results(gpu):
     for name in ('P', 'F_p', 'L_p', 'xi_sl', 'gamma_sl'):
         assert np.array_equal(a.get_field(name), b.get_field(name)), name
     print('autotune candidates (blocks/SM, chunks, ms):', cands, 'chosen', tuning['chosen'])
+    a.close()
+    b.close()
+
+
+def test_autotune_of_a_one_launch_grid(gpu):
+    """Evaluations that run as one launch have no variants and chunks to choose from: no candidates,
+    the settings as they were, and the run as the untuned one."""
+    import torch
+    limit = 2 * 128 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert np.prod(ONE_LAUNCH) <= limit < np.prod(LISTS)
+    a, sa, _ = _run(None, 2, ONE_LAUNCH)
+    b, sb, tuning = _run(1, 2, ONE_LAUNCH)
+    assert tuning == {'candidates': [], 'chosen': a.tuning()}
+    assert all(np.array_equal(x.P_av, y.P_av) for x, y in zip(sa, sb))
+    assert np.array_equal(a.get_field('xi_sl'), b.get_field('xi_sl'))
     a.close()
     b.close()
 
