@@ -6,19 +6,28 @@ from damask_b200 import synthetic, workloads
 from damask_b200.batch import DeviceBatch
 from damask_b200.grid import SpectralBasic, run_load_cases
 
+from test_stress_forms import phase_of
+
 pytestmark = pytest.mark.gpu
 
-# two resident blocks per SM: 148 x 2 x 128 = 37888 voxels, half of it at 48 systems
-AT_LIMIT, BEYOND = (64, 37, 16), (64, 37, 17)
+def at_limit(ns, beyond=0):
+    """A grid of the one-launch limit, two resident blocks of 128 threads (64 at 48 systems) on every SM, or one
+    layer more."""
+    import torch
+    sm = torch.cuda.get_device_properties(0).multi_processor_count
+    return (sm // 4, 64, (16 if ns <= 24 else 8) + beyond) if sm % 4 == 0 else (sm, 32, (8 if ns <= 24 else 4) + beyond)
 
 
-@pytest.mark.parametrize('cells,phase', [((1, 1, 1), 'fcc_al'), (AT_LIMIT, 'fcc_al'), (BEYOND, 'fcc_al'), ((8, 37, 64), 'bcc_48'),
-                                         ((9, 37, 64), 'bcc_48')])
-def test_one_launch_against_the_passes(gpu, cells, phase):
+@pytest.mark.parametrize('size,phase', [('one', 'fcc12'), ('limit', 'fcc12'), ('beyond', 'fcc12'), ('limit', 'bcc48'),
+                                        ('beyond', 'bcc48'), ('small', 'bcc12ns'), ('small', 'bcc24ns'), ('small', 'fcc18'),
+                                        ('small', 'fcc15'), ('beyond', 'bcc12ns')])
+def test_one_launch_against_the_passes(gpu, size, phase):
     """A batch runs the passes over lists at every size: two increments agree with the context's own."""
+    ns = int(phase[3:5])
+    cells = {'one': (1, 1, 1), 'small': (7, 6, 5)}.get(size) or at_limit(ns, int(size == 'beyond'))
     h = 1.0e-3 / max(cells)
     rve = synthetic.voronoi_rve(cells, tuple(h * c for c in cells), 7, 2)
-    job = (rve, getattr(workloads, phase)(), workloads.tension_x(60.0, 60), workloads.numerics_default())
+    job = (rve, phase_of(phase), workloads.tension_x(60.0, 60), workloads.numerics_default())
     db = DeviceBatch([job], max_increments=2)
     db.run_native()
     s = SpectralBasic(rve.cells, rve.size, rve.material, rve.quaternions, job[1], job[3])
@@ -33,8 +42,9 @@ def test_one_launch_against_the_passes(gpu, cells, phase):
     db.close()
 
 
-@pytest.mark.parametrize('cells', [(2, 2, 2), BEYOND])
-def test_failed_sweep_keeps_the_stress(gpu, cells):
+@pytest.mark.parametrize('beyond', [False, True])
+def test_failed_sweep_keeps_the_stress(gpu, beyond):
+    cells = at_limit(12, 1) if beyond else (2, 2, 2)
     num = workloads.numerics_default()
     rve = synthetic.voronoi_rve(cells, workloads.SIZE_1MM, 2, 0)
     num.N_iter_Lp_max = 1
