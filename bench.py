@@ -40,7 +40,8 @@ def constitutive_flops(ns: int, newton: float, state: float, updates: float) -> 
     (FMA = 2): per residual evaluation (Newton iteration) 173 + 40 Ns; per Newton step (the
     five-unknown system: assembly, QR, back-substitution; one per non-final Newton iteration)
     800 + 65 Ns; per state iteration (stress start/finish, hardening, damped update)
-    410 + 86 Ns; per substep start (kinetics and hardening) 89 Ns."""
+    410 + 86 Ns; per substep start (kinetics and hardening) 89 Ns.  The counted FP64 operations of a
+    32^3 cut with 24 systems are 5.4 % above it (profiles/constitutive_fp64_flops_32cubed_bcc24.txt)."""
     steps = max(newton - state, 0.0)
     return newton * (173 + 40 * ns) + steps * (800 + 65 * ns) + state * (410 + 86 * ns) + updates * (89 * ns)
 
@@ -48,10 +49,10 @@ def constitutive_flops(ns: int, newton: float, state: float, updates: float) -> 
 # DRAM bytes that one stress and one control launch move per voxel of a full pass, by slip-system
 # count, from the ncu captures summarised in profiles/constitutive_passes_96x96x64_bcc24.txt (24
 # systems: mean of the first pass, stress 1.11 kB and control 1.77 kB, and the second, 0.92 and 2.61 kB)
-# and profiles/constitutive_passes_64cubed_bcc48.txt (48 systems, before the start state of an
-# evaluation was no longer stored: stress 794 B, control 4 840 B); a material-point update runs one such
-# pass per state iteration
-TRAFFIC_BYTES_PER_PASS = {24: 3205, 48: 5634}
+# and profiles/constitutive_passes_64cubed_bcc48_five_unknown.txt (48 systems, the same mean: first
+# pass 1.58 and 3.42 kB, second 1.19 and 5.14 kB); a material-point update runs one such pass per state
+# iteration
+TRAFFIC_BYTES_PER_PASS = {24: 3205, 48: 5665}
 
 # the 48-system RVE's window inside the default bench line (5.7 s per increment at 256^3)
 BCC48_WARMUP, BCC48_STEPS = 3, 3
@@ -520,10 +521,10 @@ def measure(workload, steps, warmup, world, rank, local, cells, solver, derivati
         'flops_per_update': flops / max(1, mx['updates']),
         'flop_source': 'static FP64 count of the kernels times the counted Newton / state iterations',
         'traffic': traffic * mx['N'] if traffic else None,
-        'traffic_source': f'ncu DRAM bytes of a stress and a control launch per voxel and pass ({ns} systems; 24: mean of the '
-                          'first two passes at 96x96x64, 48: at 64^3 with the start state still stored), '
+        'traffic_source': f'ncu DRAM bytes of a stress and a control launch per voxel and pass ({ns} systems; mean of the '
+                          'first two passes, 24: at 96x96x64, 48: at 64^3), '
                           'times the passes (state iterations) per update and the voxels of one evaluation; '
-                          'the begin kernel is not included',
+                          'the begin and restart kernels are not included',
         'avg_launch_ms': avg_launch_ms,
         'hbm': {'achieved': achieved_gbs, 'peak': peaks['hbm_gbs'], 'unit': 'GB/s', 'frac': achieved_gbs / peaks['hbm_gbs'],
                 'peak_source': peaks['source'], 'bytes_per_update': bpu},

@@ -3,11 +3,13 @@
 //  constitutive_begin_kernel  every voxel: fused field update F <- F - r, phase restore
 //                             (mechanical_restore), substep set-up, then control up to
 //                             the first integrateStress.
+//  constitutive_restart_kernel the same in later evaluations of an increment.
 //  constitutive_stress_kernel every voxel of the list: one integrateStress (the Newton
 //                             loop; compute bound, register resident)
 //  constitutive_control_kernel every voxel of the list: state update and substep control
 //                             up to the next integrateStress (memory bound, high
 //                             occupancy); voxels that continue are appended to the next list.
+//  constitutive_fused_kernel  all of these for a small grid, in one launch.
 #include "kernels.cuh"
 #include "constitutive.cuh"
 
@@ -143,7 +145,7 @@ __device__ __forceinline__ bool begin_voxel(const PhaseConst<NS>& pc, const doub
       bad = dot_state_slots<NS>(pc, hs, s0, [&](int i) { return f.state0[i * N + v]; }, xs, nullptr, 0);
       if (bad) {
         xs[0] = nan("");
-        if (w.dot0_nan) *w.dot0_nan = 1;
+        *w.dot0_nan = 1;
       }
 #pragma unroll 12
       for (int i = 0; i < NST; ++i) w.dot0[i * N + v] = xs[i * pass_threads<NS>()];
@@ -269,7 +271,9 @@ constitutive_begin_kernel(const __grid_constant__ PhaseConst<NS> pc, const __gri
 
 // The same once the increment-start rates are stored and none of them is NaN (use_dot0 of
 // begin_voxel): no kinetics, no hardening and no slots, so the kernel streams its planes at full
-// occupancy.
+// occupancy.  Begin kernel reading the rates back -> this, an evaluation of 12 systems: 128^3 4 x 222 -> 4 x 49 us,
+// 64^3 4 x 55 -> 4 x 13 us.  Batches, and evaluations after a checkpoint's restoration or a batch solution,
+// do not know whether a rate is NaN and take the begin kernel.
 template <int NS>
 __global__ void __launch_bounds__(256)
 constitutive_restart_kernel(const __grid_constant__ Numerics nm, const __grid_constant__ Fields f,
@@ -548,7 +552,12 @@ cudaError_t launch_fused_as(const PhaseConst<NS>& pc, const Numerics& nm, const 
 }
 }  // namespace
 
-// voxels up to which an evaluation runs as one launch: two resident blocks on every SM
+// Voxels up to which an evaluation runs as one launch: two resident blocks on every SM, so that no block
+// waits for another.  Evaluations of one increment over lists / in one launch, at the limit: 12 systems 3.97 /
+// 2.41 ms, 24 systems 11.07 / 6.04 ms, 48 systems 17.40 / 12.57 ms, 12 systems in the general form 11.72 / 6.45
+// ms; at an eighth of it 1.82, 1.80, 1.35 and 2.38 to 1.  6 % beyond it the last blocks wait and the gain falls to 1.14,
+// 1.30, 1.43 and 1.57, at twice the limit 1.26, 1.43, 1.05 and 1.34: the line is on the safe side, lists are
+// not measured faster below twice of it.
 int64_t fused_voxels(int ns, int nsm) { return int64_t(nsm) * 2 * (ns > 24 ? 64 : PASS_THREADS); }
 
 template <int NS>

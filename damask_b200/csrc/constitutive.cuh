@@ -27,8 +27,9 @@
 // lives in HBM planes (PassWork), so the large per-system arrays of the state
 // iteration are never live during the Newton loop; all indexing into register
 // arrays is static, and the 9x9 Newton system, a rank-6 update of the identity, is
-// solved through its 6x6 Woodbury form by Householder QR (no data-dependent row
-// exchange, so the matrix stays in registers).
+// solved through its 6x6 Woodbury form, five unknowns in phases without non-Schmid
+// terms, by Householder QR (no data-dependent row exchange, so the matrix stays in
+// registers).  Small grids run all of it in one launch (constitutive_fused_kernel).
 #pragma once
 #include "dmk_device.cuh"
 
@@ -113,7 +114,7 @@ __device__ __forceinline__ bool qr_solve(double* A, double* b) {
 // thread's slots (stride: the block's threads): 1/xi (NS), the Newton weights (NS; without non-Schmid
 // terms also K, at least 30), A = F Fp0^-1 (9) and, where they fit, the last accepted Lp (9) and the
 // Newton step (9), which stay in local memory otherwise: the L1 that the slots leave is too small for
-// it, so every read of it goes to L2 (measured).  Blocks of 192 threads where those of 128 leave no room for Lp.
+// it, so every read of it goes to L2 (measured).
 template <int NS, bool SCHMID, int MINB>
 struct StressShape {
   static constexpr size_t consts = NS * sizeof(StressConst<SCHMID>) + 1024;   // with the system's 1 KB per block
@@ -121,9 +122,8 @@ struct StressShape {
   static constexpr bool fits(int slots, int threads, int blocks) {
     return blocks * (consts + sizeof(double) * slots * threads) <= 228 * 1024;
   }
-  static constexpr bool wide = NS <= 24 && MINB == 3 && !fits(base + 9, 128, 3) && fits(base + 9, 192, 2);
-  static constexpr int threads = NS > 24 ? 64 : wide ? 192 : 128;
-  static constexpr int blocks = NS > 24 ? 3 : wide ? 2 : MINB;
+  static constexpr int threads = NS > 24 ? 64 : 128;
+  static constexpr int blocks = NS > 24 ? 3 : MINB;
   static constexpr bool lo_shared = fits(base + 9, threads, blocks);
   static constexpr bool dl_shared = fits(base + 18, threads, blocks);
   static constexpr int slots = base + (lo_shared ? 9 : 0) + (dl_shared ? 9 : 0);
@@ -373,11 +373,12 @@ __device__ int integrate_stress(const PhaseConst<NS>& pc, const SysConst* __rest
 // The u-u part of K is symmetric, so a system adds 15 + 15 products to it instead of 36 to C6, and dLp needs
 // no second pass over the systems.  What bounds the kernel is the FP64 instructions of this function and
 // the latency of their chains at twelve warps per SM (more warps have no registers), then every memory
-// round trip that they cannot hide: all of a voxel's loads are issued at once (stress_voxel), and nothing
-// of the loop lives in memory (spills and planes of the Newton step went to L2: the slots leave little of
-// L1).  Stress kernels of one increment, general form with its loads one after the other -> this: 24
-// systems at 128^3 147 -> 94 ms, 48 systems at 40^3 17.5 -> 9.7 ms, 12 systems at 64^3 9.5 -> 6.8 ms;
-// FP64 pipe 35 -> 51 % busy, long-scoreboard stalls per issue 2.0 -> 0.45.
+// round trip that they cannot hide: all of a voxel's loads are issued at once (stress_voxel), and of the
+// loop only the Newton step, where it does not fit into the slots, lives in memory (spills and planes of
+// it went to L2: the slots leave little of L1).  Stress kernels of one increment, general form with its
+// loads one after the other -> this: 24 systems at 128^3 147 -> 94 ms, 48 systems at 40^3 17.5 -> 9.7 ms, 12
+// systems at 64^3 9.5 -> 6.8 ms.  First full pass at 24 systems (64^3 -> 96x96x64): FP64 pipe 35 -> 46 %
+// busy, long-scoreboard stalls per issue 2.0 -> 0.7.
 template <int NS, class Shape>
 __device__ int integrate_stress(const PhaseConst<NS>& pc, const SchmidConst* __restrict__ sc, const Numerics& nm,
                                 const double* F, const double* Fp0, const double* Fp0g, int64_t N, double* xs, double dt,
@@ -671,8 +672,9 @@ __device__ void advance(const PhaseConst<NS>& pc, const double* __restrict__ hs,
                         int64_t adg_stride) {
   constexpr int NST = 2 * NS;
   const int64_t N = f.N;
-  // every control step shrinks the substep or advances stepFrac; the bound only
-  // guards against numerics (r_cutback >= 1) under which the reference loops forever
+  // every control step shrinks the substep or advances stepFrac; the bound only guards against
+  // numerics (r_cutback >= 1) under which the reference loops forever, within one call (the calls of
+  // an evaluation: Numerics::max_passes)
   for (int guard = 0; c.phase != PH_STRESS && c.phase != PH_DONE; ++guard) {
     if (guard > 4096) { c.status = 3; c.phase = PH_DONE; break; }
     if (c.phase == PH_CTRL) {

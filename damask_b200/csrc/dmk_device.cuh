@@ -91,7 +91,7 @@ struct PassWork {
   double* dot0;    // 2 NS: dotState at the increment-start stress and state (S0, state0)
   double* sub;     // 2: stepFrac (subFrac), step (subStep; negative: VoxelCtl::from_start)
   int* ctl;        // 6: phase, status, state iteration, substeps, state iterations total, Newton total
-  int* dot0_nan;   // set when an increment-start rate is NaN (null in batches)
+  int* dot0_nan;   // set when an increment-start rate is NaN
   int* list_out;   // voxels that continue into the next pass
   int* count_out;  // number of entries appended to list_out
 };

@@ -274,8 +274,8 @@ dPdF_kernel(const __grid_constant__ PhaseConst<NS> pc, const __grid_constant__ F
 constexpr int TSUM_THREADS = 256, TSUM_BLOCKS = 1184;
 
 // grid.y: nine components of the 81 each, summed together; one block for all of them was 81 reductions one
-// after the other, each a memory round trip and two barriers (45 us whatever the size, 154 us at 64^3).  The
-// sums keep their order.
+// after the other, each a memory round trip and two barriers.  8^3 46 -> 3 us, 32^3 54 -> 7 us, 64^3 156 ->
+// 42 us, 128^3 369 -> 217 us.  The sums keep their order.
 constexpr int TSUM_COMPONENTS = 9;
 __global__ void __launch_bounds__(TSUM_THREADS)
 tangent_sum_kernel(const double* __restrict__ planes, const double* __restrict__ norms, int64_t first, int64_t count,

@@ -182,7 +182,7 @@ struct AASlots {
   int slot[AA_CHUNK];
   int write;                   // this launch writes dR and dX of the new slot
 };
-struct AAUpdate {              // X <- X - R - sum_q gamma_q (dX[slot_q] - dR[slot_q])
+struct AAUpdate {              // X <- X - R - sum_q gamma_q dX[slot_q], where dX holds dX - dR by then
   int n;
   int slot[AA_MAX];
   double gamma[AA_MAX];
